@@ -32,8 +32,10 @@ namespace gcge {
 __global__ void __launch_bounds__(256)
 k_gram(int n, int m, int w, const double *__restrict__ Q, int ldq, const double *__restrict__ P,
        int ldp, double *__restrict__ part, int rows_per_chunk);
-__global__ void k_reduce_chunks(const double *__restrict__ part, int chunks, int m, int w,
-                                double *__restrict__ C, int ldc);
+__global__ void __launch_bounds__(256)
+k_reduce_chunks(const double *__restrict__ part, int chunks, int m, int w,
+                double *__restrict__ C, int ldc);
+int reduce_chunks_blocks(int chunks, int outputs, int sms);
 }  // namespace gcge
 
 namespace {
@@ -121,7 +123,7 @@ extern "C" int GCGE_GramNoAlloc(int n, int m, int w, const double *Q, int ldq, c
     const dim3 grid(nchunks, (m + kTile - 1) / kTile, (w + kTile - 1) / kTile);
     gcge::k_gram<<<grid, 256, 0, s>>>(n, m, w, Q, ldq, P, ldp, scratch, rpc);
     const int tot = m * w;
-    gcge::k_reduce_chunks<<<std::max(1, std::min((tot + 255) / 256, 4 * sms)), 256, 0, s>>>(
+    gcge::k_reduce_chunks<<<gcge::reduce_chunks_blocks(nchunks, tot, sms), 256, 0, s>>>(
         scratch, nchunks, m, w, C, ldc);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
