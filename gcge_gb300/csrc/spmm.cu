@@ -28,7 +28,13 @@ int spmm_blocks(const SellPattern &pat) {
 }
 
 // ---------------------------------------------------------------- kernels
-template <typename T, int K>
+// K accumulators per lane for k columns, KLO <= k <= K: columns below KLO need
+// no test.  The FP64 units bound the FP64 kernels (two FMAs per clock and SM)
+// and a predicated-off FMA costs as much as a live one, so the widths are
+// closely spaced: 20 columns of a 27-point 64^3 operator took 310 us with 24
+// accumulators (229 us is the FP64 rate), and dropping the tests below KLO
+// took 40 columns of a 7-point 128^3 operator from 1.025 to 0.953 ms.
+template <typename T, int K, int KLO>
 __global__ void __launch_bounds__(kSpmmThreads)
 k_spmm(const long long *__restrict__ sp, const int *__restrict__ col, const T *__restrict__ val,
        int n, int nslices, const T *__restrict__ X, int ldx, T *__restrict__ Y, int ldy, int k) {
@@ -45,17 +51,17 @@ k_spmm(const long long *__restrict__ sp, const int *__restrict__ col, const T *_
         const T *xj = X + j;
 #pragma unroll
         for (int c = 0; c < K; ++c)
-            if (c < k) acc[c] = fma(a, __ldg(xj + (size_t)c * ldx), acc[c]);
+            if (c < KLO || c < k) acc[c] = fma(a, __ldg(xj + (size_t)c * ldx), acc[c]);
     }
     const int row = slice * 32 + lane;
     if (row < n) {
 #pragma unroll
         for (int c = 0; c < K; ++c)
-            if (c < k) Y[row + (size_t)c * ldy] = acc[c];
+            if (c < KLO || c < k) Y[row + (size_t)c * ldy] = acc[c];
     }
 }
 
-template <int K>
+template <int K, int KLO>
 __global__ void __launch_bounds__(kSpmmThreads)
 k_residual(const long long *__restrict__ sa, const int *__restrict__ ca,
            const double *__restrict__ va, const long long *__restrict__ sb,
@@ -84,13 +90,13 @@ k_residual(const long long *__restrict__ sa, const int *__restrict__ ca,
             const double *xj = X + __ldg(ca + e);
 #pragma unroll
             for (int c = 0; c < K; ++c)
-                if (c < k) acc[c] = fma(v, __ldg(xj + (size_t)c * ldx), acc[c]);
+                if (c < KLO || c < k) acc[c] = fma(v, __ldg(xj + (size_t)c * ldx), acc[c]);
         }
     }
     if (row < n) {
 #pragma unroll
         for (int c = 0; c < K; ++c)
-            if (c < k) ax[row + (size_t)c * ldo] = acc[c];
+            if (c < KLO || c < k) ax[row + (size_t)c * ldo] = acc[c];
     }
 #pragma unroll
     for (int c = 0; c < K; ++c) acc[c] = 0.0;
@@ -101,23 +107,23 @@ k_residual(const long long *__restrict__ sa, const int *__restrict__ ca,
                 const double *xj = X + __ldg(cb + e);
 #pragma unroll
                 for (int c = 0; c < K; ++c)
-                    if (c < k) acc[c] = fma(v, __ldg(xj + (size_t)c * ldx), acc[c]);
+                    if (c < KLO || c < k) acc[c] = fma(v, __ldg(xj + (size_t)c * ldx), acc[c]);
             }
         } else if (row < n) {  // B = I
 #pragma unroll
             for (int c = 0; c < K; ++c)
-                if (c < k) acc[c] = X[row + (size_t)c * ldx];
+                if (c < KLO || c < k) acc[c] = X[row + (size_t)c * ldx];
         }
     }
     if (row < n) {
 #pragma unroll
         for (int c = 0; c < K; ++c)
-            if (c < k) bx[row + (size_t)c * ldo] = acc[c];
+            if (c < KLO || c < k) bx[row + (size_t)c * ldo] = acc[c];
     }
 #pragma unroll
     for (int c = 0; c < K; ++c) {
         double v = 0.0;
-        if (row < n && c < k) {
+        if (row < n && (c < KLO || c < k)) {
             const double r = fma(-slam[c], acc[c], ax[row + (size_t)c * ldo]);
             v = r * r;
         }
@@ -134,19 +140,29 @@ k_residual(const long long *__restrict__ sa, const int *__restrict__ ca,
 }
 
 // ---------------------------------------------------------------- dispatch
-#define GCGE_K_DISPATCH(kk, BODY)                          \
-    do {                                                   \
-        if ((kk) <= 4) { constexpr int KT = 4; BODY; }        \
-        else if ((kk) <= 8) { constexpr int KT = 8; BODY; }   \
-        else if ((kk) <= 16) { constexpr int KT = 16; BODY; } \
-        else if ((kk) <= 24) { constexpr int KT = 24; BODY; } \
-        else if ((kk) <= 32) { constexpr int KT = 32; BODY; } \
-        else { constexpr int KT = 40; BODY; }                 \
+#define GCGE_K_DISPATCH(kk, BODY)                                                 \
+    do {                                                                          \
+        if ((kk) <= 2) { constexpr int KT = 2, KL = 1; BODY; }                       \
+        else if ((kk) <= 4) { constexpr int KT = 4, KL = 3; BODY; }                  \
+        else if ((kk) <= 6) { constexpr int KT = 6, KL = 5; BODY; }                  \
+        else if ((kk) <= 8) { constexpr int KT = 8, KL = 7; BODY; }                  \
+        else if ((kk) <= 10) { constexpr int KT = 10, KL = 9; BODY; }                \
+        else if ((kk) <= 12) { constexpr int KT = 12, KL = 11; BODY; }               \
+        else if ((kk) <= 14) { constexpr int KT = 14, KL = 13; BODY; }               \
+        else if ((kk) <= 16) { constexpr int KT = 16, KL = 15; BODY; }               \
+        else if ((kk) <= 18) { constexpr int KT = 18, KL = 17; BODY; }               \
+        else if ((kk) <= 20) { constexpr int KT = 20, KL = 19; BODY; }               \
+        else if ((kk) <= 24) { constexpr int KT = 24, KL = 21; BODY; }               \
+        else if ((kk) <= 28) { constexpr int KT = 28, KL = 25; BODY; }               \
+        else if ((kk) <= 32) { constexpr int KT = 32, KL = 29; BODY; }               \
+        else if ((kk) <= 36) { constexpr int KT = 36, KL = 33; BODY; }               \
+        else { constexpr int KT = 40, KL = 37; BODY; }                               \
     } while (0)
 
 constexpr int kMaxChunk = 40;
 
-// Register width (accumulators per lane) GCGE_K_DISPATCH gives kc columns.
+// Width class of a launch of kc columns for the tuner: candidates within one
+// class differ too little in registers to be worth timing.
 static int spmm_dispatch_width(int kc) {
     return kc <= 4 ? 4 : kc <= 8 ? 8 : kc <= 16 ? 16 : kc <= 24 ? 24 : kc <= 32 ? 32 : 40;
 }
@@ -161,7 +177,7 @@ static void spmm_split(const SellPattern &pat, const T *val, const T *X, int ldx
     const int blocks = spmm_blocks(pat);
     for (int c0 = 0; c0 < k; c0 += chunk) {
         const int kc = std::min(chunk, k - c0);
-        GCGE_K_DISPATCH(kc, (k_spmm<T, KT><<<blocks, kSpmmThreads, 0, st>>>(
+        GCGE_K_DISPATCH(kc, (k_spmm<T, KT, KL><<<blocks, kSpmmThreads, 0, st>>>(
                                 pat.slice_ptr.p, pat.col.p, val, pat.n, pat.nslices,
                                 X + (size_t)c0 * ldx, ldx, Y + (size_t)c0 * ldy, ldy, kc)));
         GCGE_CHECK_LAUNCH();
@@ -176,7 +192,7 @@ static void spmm_split(const SellPattern &pat, const T *val, const T *X, int ldx
 // (entries per row, locality of its columns) and the device, so the tuner
 // measures it.  Candidates split k columns into p equal launches, p from
 // ceil(k / 40) up while a launch keeps at least 8 columns; of the p that give
-// the same register width only the smallest is kept (more launches of the
+// the same width class only the smallest is kept (more launches of about the
 // same width only re-read the matrix).
 std::vector<int> spmm_split_candidates(int k) {
     std::vector<int> out;
@@ -314,7 +330,7 @@ int residual_norms(const SellPattern &pa, const double *va, const SellPattern *p
                  "residual_norms: patterns differ in size");
     const int blocks = spmm_blocks(pa);
     if (k <= 0) return 0;
-    GCGE_K_DISPATCH(k, (k_residual<KT><<<blocks, kSpmmThreads, 0, st>>>(
+    GCGE_K_DISPATCH(k, (k_residual<KT, KL><<<blocks, kSpmmThreads, 0, st>>>(
                            pa.slice_ptr.p, pa.col.p, va, pb ? pb->slice_ptr.p : nullptr,
                            pb ? pb->col.p : nullptr, vb, pa.n, pa.nslices, X, ldx, lam, k,
                            partial, kmax, ax, bx, ldo)));
