@@ -224,16 +224,19 @@ k_jacobi32(int s, const double *__restrict__ M, int ldm, float4 *__restrict__ lo
 // pair slot k of round r is (P_r[k], P_r[m - 1 - k]); after m - 1 rounds P is
 // the identity again.  CTA c owns the slots [c np / kJC, (c + 1) np / kJC) and
 // holds the two full rows (m floats each) of each of its slots.  A round:
-//   (a) every CTA computes the rotations of its slots and writes them into the
-//       round table of every CTA of the cluster;
-//   (b) after a cluster barrier, each CTA updates every 2x2 block (own slot i,
-//       any slot j) of its rows, A <- J^T A J, and writes the new rows into
-//       the other row buffer at the slots they hold in the next round, which
-//       for at most two rows per CTA is in the neighbouring CTA's shared
-//       memory;
-//   (c) a second cluster barrier makes the next buffers complete.
-// Rotations and the stopping test are those of k_jacobi32; every CTA sums the
-// per-CTA off-diagonal masses in the same order, so all take the same decision.
+//   (a) every CTA computes all np rotations from the table of the pairs'
+//       a_pp, a_qq and a_pq that the previous round left in its shared memory;
+//   (b) it updates every 2x2 block (own slot i, any slot j) of its rows,
+//       A <- J^T A J, writes the new rows into the other row buffer at the
+//       slots they hold in the next round, which for at most two rows per CTA
+//       is in the neighbouring CTA's shared memory, and the entries that the
+//       next round's rotations need into every CTA's table;
+//   (c) one cluster barrier makes the next buffers and tables complete.
+// The round is bound by the latency of its serial chain, of which a barrier is
+// the longest link: computing the rotations eight times over costs less than
+// the second barrier that sharing them took.
+// The stopping test is that of k_jacobi32; every CTA sums the per-CTA
+// off-diagonal masses in the same order, so all take the same decision.
 constexpr int kJC = 8;
 // Smaller matrices use the one-CTA kernel.  Measured on GB300 (RR-shaped
 // matrices, kernel time): s = 64, 80: one CTA 480, 609 us, cluster 510, 652 us;
@@ -245,35 +248,38 @@ __host__ __device__ inline int jc_slots(int np) { return (np + kJC - 1) / kJC; }
 
 size_t jacobi_cluster_smem_bytes(int s) {
     const int m = jac_m(s), np = m / 2, ks = jc_slots(np);
-    return (size_t)2 * np * sizeof(float4) + (size_t)2 * 2 * ks * m * sizeof(float) +
-           (size_t)2 * kJC * 2 * sizeof(float) + 64;
+    return (size_t)np * sizeof(float4) + (size_t)2 * 2 * ks * m * sizeof(float) +
+           (size_t)2 * kJC * 2 * sizeof(float) + (size_t)2 * 3 * np * sizeof(float) + 64;
 }
 
-// index at position i of the circle arrangement after r rounds
+// index at position i < m1 + 1 of the circle arrangement after r < m1 rounds
 __device__ __forceinline__ int circle_index(int i, int r, int m1) {
     if (i == 0) return 0;
-    int v = i - 1 - r;
-    v %= m1;
-    if (v < 0) v += m1;
-    return 1 + v;
+    const int v = i - 1 - r;
+    return 1 + (v < 0 ? v + m1 : v);
 }
 
 // CTA owning slot k (slots [c np / kJC, (c + 1) np / kJC) belong to CTA c)
 __device__ __forceinline__ int slot_owner(int k, int np) { return ((k + 1) * kJC - 1) / np; }
 
 __global__ void __launch_bounds__(kJacobiThreads, 1)
-k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float4 *__restrict__ log,
+k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restrict__ log,
                    int max_rounds, int *__restrict__ info) {
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     extern __shared__ __align__(16) unsigned char jsm[];
     const int m = jac_m(s), np = m / 2, ks = jc_slots(np), m1 = m - 1;
-    float4 *table = reinterpret_cast<float4 *>(jsm);  // [2][np]
-    float *rows = reinterpret_cast<float *>(table + 2 * np);  // [2][2 ks][m]
-    float *red = rows + (size_t)2 * 2 * ks * m;                 // [2][kJC][2]
+    float4 *tab = reinterpret_cast<float4 *>(jsm);          // [np]: c, s, p, q of the round
+    float *rows = reinterpret_cast<float *>(tab + np);      // [2][2 ks][m]
+    float *red = rows + (size_t)2 * 2 * ks * m;               // [2][kJC][2]
+    float *piv = red + 2 * kJC * 2;                          // [2][3][np]: a_pp, a_qq, a_pq
     __shared__ float wsum[kJacobiThreads / 32][2];
     __shared__ int stop;
-    __shared__ float *s_dst[2 * kJacMaxLocal];  // next-round rows of each local slot
+    // each local row in the next round: where it is stored, its slot (2 k for
+    // the top row of slot k, 2 k + 1 for the bottom one), and for a top row its
+    // partner's index
+    __shared__ float *s_dst[2 * kJacMaxLocal];
+    __shared__ int s_slot[2 * kJacMaxLocal], s_partner[2 * kJacMaxLocal];
     const size_t bufsz = (size_t)2 * ks * m;
     const int k0 = (rank * np) / kJC, k1 = ((rank + 1) * np) / kJC, nloc = k1 - k0;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
@@ -287,6 +293,20 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float4 *__restr
         rows[(size_t)lr * m + y] = v;
     }
     cl.sync();  // every CTA of the cluster runs before any remote access
+    // entry `what` (0 a_pp, 1 a_qq, 2 a_pq) of slot k, into every CTA's table
+    auto share = [&](int parity, int what, int k, float v) {
+        float *at = piv + ((size_t)parity * 3 + what) * np + k;
+#pragma unroll
+        for (int c = 0; c < kJC; ++c) *cl.map_shared_rank(at, c) = v;
+    };
+    for (int ls = t; ls < nloc; ls += blockDim.x) {
+        const int k = k0 + ls;
+        const float *top = rows + (size_t)(2 * ls) * m;
+        share(0, 0, k, top[k]);
+        share(0, 1, k, top[m + m - 1 - k]);
+        share(0, 2, k, top[m - 1 - k]);
+    }
+    cl.sync();
     int cur = 0, round = 0, sweep = 0, converged = 0;
     for (sweep = 0; sweep < kMaxSweeps && round + m1 <= max_rounds; ++sweep) {
         // off-diagonal mass at the start of the sweep (P = identity again)
@@ -340,49 +360,47 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float4 *__restr
         }
         for (int r = 0; r < m1; ++r) {
             const float *R = rows + cur * bufsz;
-            float4 *tab = table + (round & 1) * np;
-            // (a) rotations of the local slots, into every CTA's round table
-            for (int ls = t; ls < nloc; ls += blockDim.x) {
-                const int k = k0 + ls;
+            const int par = round & 1, rn = r + 1 == m1 ? 0 : r + 1;
+            // (a) the round's rotations, from the pairs' entries
+            for (int k = t; k < np; k += blockDim.x) {
                 const int p = circle_index(k, r, m1), q = circle_index(m - 1 - k, r, m1);
                 float c = 1.0f, sv = 0.0f;
                 if (p < s && q < s) {
-                    const float app = R[(size_t)(2 * ls) * m + p];
-                    const float aqq = R[(size_t)(2 * ls + 1) * m + q];
-                    const float apq = R[(size_t)(2 * ls) * m + q];
+                    const float *pv = piv + (size_t)par * 3 * np + k;
+                    const float app = pv[0], aqq = pv[np], apq = pv[2 * np];
                     const float thr = kRotTol * sqrtf(fabsf(app) * fabsf(aqq));
                     if (fabsf(apq) > thr && fabsf(apq) > 1e-30f) {
+                        // (an infinite tau^2 gives the rotation 0, as it should)
                         const float tau = (aqq - app) / (2.0f * apq);
-                        const float tt =
-                            (tau >= 0.0f ? 1.0f : -1.0f) / (fabsf(tau) + hypotf(1.0f, tau));
+                        const float tt = (tau >= 0.0f ? 1.0f : -1.0f) /
+                                         (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.0f)));
                         c = rsqrtf(1.0f + tt * tt);
                         sv = tt * c;
                     }
                 }
-                const float4 e = make_float4(c, sv, __int_as_float(p), __int_as_float(q));
-                for (int cc = 0; cc < kJC; ++cc) *cl.map_shared_rank(tab + k, cc) = e;
-                log[(size_t)round * np + k] = e;
-                // next-round positions of the slot's two rows (circle method)
-                int kt, st_, kb, sb;
-                if (np == 1) {
-                    kt = 0, st_ = 0, kb = 0, sb = 1;
-                } else {
-                    if (k == 0) kt = 0, st_ = 0;
-                    else if (k <= np - 2) kt = k + 1, st_ = 0;
-                    else kt = np - 1, st_ = 1;
-                    if (k == 0) kb = 1, sb = 0;
-                    else kb = k - 1, sb = 1;
-                }
-                const int ot = slot_owner(kt, np), ob = slot_owner(kb, np);
-                const size_t nb = (size_t)(cur ^ 1) * bufsz;
-                float *dt = rows + nb + (size_t)(2 * (kt - (ot * np) / kJC) + st_) * m;
-                float *db = rows + nb + (size_t)(2 * (kb - (ob * np) / kJC) + sb) * m;
-                s_dst[2 * ls] = ot == rank ? dt : cl.map_shared_rank(dt, ot);
-                s_dst[2 * ls + 1] = ob == rank ? db : cl.map_shared_rank(db, ob);
+                tab[k] = make_float4(c, sv, __int_as_float(p), __int_as_float(q));
+                if (k >= k0 && k < k1) log[(size_t)round * np + k] = make_float2(c, sv);
             }
-            cl.sync();
+            // next-round places of the local rows (circle method)
+            for (int lr = (int)blockDim.x - 1 - t; lr < 2 * nloc; lr += blockDim.x) {
+                const int k = k0 + (lr >> 1);
+                int kn, sn;
+                if (np == 1) kn = 0, sn = lr & 1;
+                else if (lr & 1) kn = k == 0 ? 1 : k - 1, sn = k == 0 ? 0 : 1;
+                else if (k == 0) kn = 0, sn = 0;
+                else if (k <= np - 2) kn = k + 1, sn = 0;
+                else kn = np - 1, sn = 1;
+                const int o = slot_owner(kn, np);
+                float *d = rows + (size_t)(cur ^ 1) * bufsz +
+                           (size_t)(2 * (kn - (o * np) / kJC) + sn) * m;
+                s_dst[lr] = o == rank ? d : cl.map_shared_rank(d, o);
+                s_slot[lr] = 2 * kn + sn;
+                s_partner[lr] = sn == 0 ? circle_index(m - 1 - kn, rn, m1) : -1;
+            }
+            __syncthreads();
             // (b) the 2x2 blocks of the local rows, written to the next buffers
             const float inv_np = 1.0f / (float)np;  // b / np exactly: the quotient's
+#pragma unroll 2
             for (int b = t; b < nloc * np; b += blockDim.x) {  // fraction is >= 0.5 / np away
                 const int li = (int)(((float)b + 0.5f) * inv_np);
                 const int j = b - li * np;
@@ -420,6 +438,15 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float4 *__restr
                 dt[qj] = o12;
                 db[pj] = o21;
                 db[qj] = o22;
+                // what the next round's rotations need of these entries
+                const int nt = s_slot[2 * li], nb = s_slot[2 * li + 1];
+                if (ki == j) {
+                    share(par ^ 1, nt & 1, nt >> 1, o11);
+                    share(par ^ 1, nb & 1, nb >> 1, o22);
+                }
+                const int pt = s_partner[2 * li], pb = s_partner[2 * li + 1];
+                if (pt == pj || pt == qj) share(par ^ 1, 2, nt >> 1, pt == pj ? o11 : o12);
+                if (pb == pj || pb == qj) share(par ^ 1, 2, nb >> 1, pb == pj ? o21 : o22);
             }
             cl.sync();
             cur ^= 1;
@@ -518,6 +545,81 @@ static void launch_rotations(int s, const float4 *log, const int *info, double *
                              cudaStream_t st) {
     k_apply_rotations<NS><<<(s + 7) / 8, 256, (size_t)8 * s * sizeof(float), st>>>(s, log, info,
                                                                                   V, ldv);
+}
+
+// The same product from the cluster kernel's log, whose rounds follow the
+// circle method: slot k's pair sits at positions k and m - 1 - k of the
+// arrangement, and between rounds every entry moves on by one position.  A
+// warp holds its row by position in registers (lane l slots [l NS, (l + 1) NS):
+// the two entries of each), rotates the slots' pairs and moves the entries, one
+// of each end to the neighbouring lanes, so that a round is a dozen dependent
+// instructions and no memory but the log (c, s per slot), which the kernel
+// reads kCircleAhead rounds ahead.  The arrangement is back at the identity
+// after whole sweeps, which is all that the log holds.  s = 180: 92 us through
+// shared memory, with the pairs' indices read from the log.
+constexpr int kCircleAhead = 4;
+template <int NS>
+__global__ void __launch_bounds__(128)
+k_apply_circle(int s, const float2 *__restrict__ log, const int *__restrict__ info,
+               double *__restrict__ V, int ldv) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row = blockIdx.x * 4 + warp;
+    if (row >= s) return;  // warp-uniform; the kernel has no block-wide barrier
+    const int m = jac_m(s), np = m / 2, rounds = info[0];
+    const int k0 = lane * NS;
+    float top[NS], bot[NS];
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        top[j] = k0 + j == row ? 1.0f : 0.0f;
+        bot[j] = m - 1 - (k0 + j) == row ? 1.0f : 0.0f;
+    }
+    float2 q[kCircleAhead][NS];
+    auto load = [&](float2 (&dst)[NS], int t) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j)
+            dst[j] = (t < rounds && k0 + j < np) ? __ldg(log + (size_t)t * np + k0 + j)
+                                                 : make_float2(1.0f, 0.0f);
+    };
+    auto step = [&](const float2 (&e)[NS]) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+            const float vt = top[j], vb = bot[j];
+            top[j] = e[j].x * vt - e[j].y * vb;
+            bot[j] = e[j].y * vt + e[j].x * vb;
+        }
+        // top k -> top k + 1, bottom k -> bottom k - 1; top 0 stays, bottom 0 ->
+        // top 1, top np - 1 -> bottom np - 1
+        const float b0 = bot[0];
+        const float from_left = __shfl_up_sync(0xffffffffu, NS == 1 && lane == 0 ? b0 : top[NS - 1], 1);
+        const float from_right = __shfl_down_sync(0xffffffffu, b0, 1);
+        const float first = top[0];
+        float nt[NS], nb[NS];
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+            nt[j] = j == 0 ? from_left : (j == 1 && lane == 0 ? b0 : top[j - 1]);
+            nb[j] = k0 + j == np - 1 ? top[j] : (j + 1 < NS ? bot[j + 1 < NS ? j + 1 : j] : from_right);
+        }
+        if (lane == 0) nt[0] = first;
+#pragma unroll
+        for (int j = 0; j < NS; ++j) top[j] = nt[j], bot[j] = nb[j];
+    };
+#pragma unroll
+    for (int g = 0; g < kCircleAhead; ++g) load(q[g], g);
+    for (int t0 = 0; t0 < rounds; t0 += kCircleAhead) {
+#pragma unroll
+        for (int g = 0; g < kCircleAhead; ++g) {
+            if (t0 + g < rounds) step(q[g]);  // warp-uniform
+            load(q[g], t0 + g + kCircleAhead);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        const int k = k0 + j;
+        if (k < np) {
+            V[row + (size_t)k * ldv] = (double)top[j];
+            if (m - 1 - k < s) V[row + (size_t)(m - 1 - k) * ldv] = (double)bot[j];
+        }
+    }
 }
 
 // Whether a cluster of kJC CTAs with the largest shared memory the cluster
@@ -689,24 +791,35 @@ int sym_eig(EigWork &wk, int s, const double *M, int ld, double *eval_host, doub
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi32_cluster, s, M, ld, wk.log.p, wk.max_rounds,
+        float2 *log = reinterpret_cast<float2 *>(wk.log.p);
+        GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi32_cluster, s, M, ld, log, wk.max_rounds,
                                      wk.info.p));
+        GCGE_CHECK_LAUNCH();
+        const int grid = (s + 3) / 4;
+        switch ((jac_m(s) / 2 + 31) / 32) {
+#define GCGE_CIRCLE_CASE(NS)                                                        \
+    case NS:                                                                        \
+        k_apply_circle<NS><<<grid, 128, 0, st>>>(s, log, wk.info.p, wk.X.p, s);      \
+        break;
+            GCGE_CIRCLE_CASE(2) GCGE_CIRCLE_CASE(3) GCGE_CIRCLE_CASE(4) GCGE_CIRCLE_CASE(5)
+            GCGE_CIRCLE_CASE(6) GCGE_CIRCLE_CASE(7) GCGE_CIRCLE_CASE(8)
+#undef GCGE_CIRCLE_CASE
+            default: throw CudaError{GCGE_ERR_TOO_LARGE, "sym_eig: size"};
+        }
     } else {
         GCGE_REQUIRE(jacobi_smem_bytes(s) <= jacobi_dyn_limit(), GCGE_ERR_TOO_LARGE,
                      "sym_eig: projected dimension exceeds the one-CTA Jacobi capacity");
         k_jacobi32<<<1, kJacobiThreads, jacobi_smem_bytes(s), st>>>(s, M, ld, wk.log.p,
                                                                     wk.max_rounds, wk.info.p);
-    }
-    GCGE_CHECK_LAUNCH();
-    switch ((jac_m(s) / 2 + 31) / 32) {
-        case 1: launch_rotations<1>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 2: launch_rotations<2>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 3: launch_rotations<3>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 4: launch_rotations<4>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 5: launch_rotations<5>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 6: launch_rotations<6>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        case 7: launch_rotations<7>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
-        default: launch_rotations<8>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+        GCGE_CHECK_LAUNCH();
+        switch ((jac_m(s) / 2 + 31) / 32) {
+            case 1: launch_rotations<1>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+            case 2: launch_rotations<2>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+            case 3: launch_rotations<3>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+            case 4: launch_rotations<4>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+            case 5: launch_rotations<5>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+            default: launch_rotations<6>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
+        }
     }
     GCGE_CHECK_LAUNCH();
     count_launch(2);
