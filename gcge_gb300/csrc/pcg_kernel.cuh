@@ -1,0 +1,1505 @@
+// Block conjugate gradient on (A + sigma B) x = b for all columns of a block
+// at once (reference BlockPCG, src/ops_lin_sol.c:140-437).
+//
+// The whole solve is ONE persistent kernel launch (cooperative grid, or one
+// thread-block cluster for small operators, below).  Each block
+// owns a contiguous range of SELL slices (balanced by stored entries) and the
+// rows they cover; the iteration runs in three phases separated by grid-wide
+// barriers:
+//   1. p = r + beta p                      (own rows; p = r on the first step)
+//   2. w = S p, partial sums of p^T w      (warp per slice, gathers p rows)
+//      -> the last block to arrive sums the partials: alpha = rho / p^T w
+//   3. x += alpha p, r -= alpha w, partial sums of r^T r
+//      -> the last block: residual norms, convergence test, beta, count
+// so nothing returns to the host between iterations.  The reference keeps a
+// compacted list of unconverged columns and runs one SpMM per contiguous run
+// of them; here a per-column `active` flag plays that role: inactive columns
+// keep x and r (alpha = 0), drop out of the sums, and a 16-byte group of
+// columns that is wholly inactive is neither gathered nor updated.
+//
+// Cross-block sums are taken by one block in a fixed order, so results are
+// deterministic for a given grid.  The shifted operator is one SELL matrix
+// S = A + sigma B on the union pattern of A and B (the reference's in-place
+// MatAxpby branch, src/ops_eig_sol_gcg.c:600-608), so each iteration streams
+// one matrix.  Vectors are slice-blocked n x kp blocks (kp = k padded to 16
+// bytes, G = kp / (16 / sizeof T) 16-byte column groups; for every 32-row
+// slice, group u of its 32 rows is one contiguous 512-byte run): a lane owns
+// a row and gathers a neighbour row as G 16-byte loads, and for a stencil the
+// 32 lanes of a warp read one or two contiguous runs per load instead of 32
+// scattered rows.  T = double (FP64 GCG) or float (mixed precision: FP32
+// values and FP32 accumulation within a block; cross-block sums in double).
+//
+// Every barrier wait is bounded (time and poll count); a wait that runs out
+// sets an error flag that makes all blocks return, and the host reports it.
+//
+// Small operators, whose steps are bound by the barriers and by the latency of
+// each phase instead, run k_pcg_small (below).
+//
+// (Included by pcg.cu and pcg_f64.cu, which instantiate it for FP32 and FP64:
+// the widths take a minute to compile.)
+#pragma once
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <mutex>
+#include <type_traits>
+
+#include "common.cuh"
+#include "pcg.cuh"
+
+namespace gcge {
+
+namespace {
+
+constexpr unsigned long long kBarrierTimeoutNs = 4000000000ull;  // 4 s
+constexpr long long kBarrierMaxPolls = 1LL << 27;
+
+// 16-byte packs of a slice-blocked block
+template <typename T>
+struct Pk;
+template <>
+struct Pk<float> {
+    static constexpr int L = 4;
+    float v[4];
+    __device__ __forceinline__ static Pk ld(const float *p) {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        return Pk{{t.x, t.y, t.z, t.w}};
+    }
+    __device__ __forceinline__ void st(float *p) const {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+};
+template <>
+struct Pk<double> {
+    static constexpr int L = 2;
+    double v[2];
+    __device__ __forceinline__ static Pk ld(const double *p) {
+        const double2 t = *reinterpret_cast<const double2 *>(p);
+        return Pk{{t.x, t.y}};
+    }
+    __device__ __forceinline__ void st(double *p) const {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+
+// Element offset of row i, 16-byte group u in a slice-blocked block of width KP.
+template <typename T, int KP>
+__device__ __forceinline__ size_t boff(int i, int u) {
+    constexpr int L = Pk<T>::L, G = KP / L;
+    return ((size_t)(i >> 5) * G + u) * (32 * L) + (size_t)(i & 31) * L;
+}
+
+// acc += sum over the lane's row of a slice of val[e] * X(col[e], :), e =
+// e0 + 32 i, i < width: the column indices and values of the next kPrefetch
+// entries are in flight while the current entry's 16-byte groups are gathered,
+// so the gathers do not wait on the matrix stream.  Groups with ga[u] false
+// are skipped.
+constexpr int kPrefetch = 2;
+template <typename T, int KP>
+__device__ __forceinline__ void gather_row(const int *__restrict__ col, const T *__restrict__ val,
+                                           long long e0, int width, const T *X,
+                                           const bool (&ga)[KP / Pk<T>::L], T (&acc)[KP]) {
+    constexpr int L = Pk<T>::L, G = KP / L;
+    int jq[kPrefetch];
+    T vq[kPrefetch];
+#pragma unroll
+    for (int d = 0; d < kPrefetch; ++d) {
+        const bool in = d < width;
+        jq[d] = in ? __ldg(col + e0 + 32LL * d) : 0;
+        vq[d] = in ? __ldg(val + e0 + 32LL * d) : T(0);
+    }
+#pragma unroll 1
+    for (int e = 0; e < width; ++e) {
+        const int j = jq[0];
+        const T v = vq[0];
+#pragma unroll
+        for (int d = 0; d + 1 < kPrefetch; ++d) {
+            jq[d] = jq[d + 1];
+            vq[d] = vq[d + 1];
+        }
+        const int en = e + kPrefetch;
+        jq[kPrefetch - 1] = en < width ? __ldg(col + e0 + 32LL * en) : 0;
+        vq[kPrefetch - 1] = en < width ? __ldg(val + e0 + 32LL * en) : T(0);
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+            if (!ga[u]) continue;
+            const Pk<T> x = Pk<T>::ld(X + boff<T, KP>(j, u));
+#pragma unroll
+            for (int q = 0; q < L; ++q) acc[u * L + q] = fma(v, x.v[q], acc[u * L + q]);
+        }
+    }
+}
+
+// The same sum for the NU column groups [U0, U0 + NU) only (all of them,
+// active or not), two matrix entries at a time (both entries' loads in
+// flight before their FMAs): the SpMM phase of wide blocks gathers a row in
+// two such halves, so that the accumulators of one half leave registers for
+// the second entry's loads (4.87 -> 4.75 s of inner solve per 128^3 solve;
+// four entries at a time: 4.81 s).
+template <typename T, int KP, int U0, int NU, int NE>
+__device__ __forceinline__ void gather_entries(const int *__restrict__ col,
+                                               const T *__restrict__ val, long long e0, int e,
+                                               const T *X, T (&acc)[NU * Pk<T>::L]) {
+    constexpr int L = Pk<T>::L;
+    int j[NE];
+    T v[NE];
+#pragma unroll
+    for (int d = 0; d < NE; ++d) {
+        j[d] = __ldg(col + e0 + 32LL * (e + d));
+        v[d] = __ldg(val + e0 + 32LL * (e + d));
+    }
+    Pk<T> x[NE][NU];
+#pragma unroll
+    for (int d = 0; d < NE; ++d)
+#pragma unroll
+        for (int u = 0; u < NU; ++u) x[d][u] = Pk<T>::ld(X + boff<T, KP>(j[d], U0 + u));
+#pragma unroll
+    for (int d = 0; d < NE; ++d)
+#pragma unroll
+        for (int u = 0; u < NU; ++u)
+#pragma unroll
+            for (int q = 0; q < L; ++q) acc[u * L + q] = fma(v[d], x[d][u].v[q], acc[u * L + q]);
+}
+template <typename T, int KP, int U0, int NU>
+__device__ __forceinline__ void gather_row_part(const int *__restrict__ col,
+                                                const T *__restrict__ val, long long e0,
+                                                int width, const T *X, T (&acc)[NU * Pk<T>::L]) {
+    int e = 0;
+#pragma unroll 1
+    for (; e + 1 < width; e += 2) gather_entries<T, KP, U0, NU, 2>(col, val, e0, e, X, acc);
+    if (e < width) gather_entries<T, KP, U0, NU, 1>(col, val, e0, e, X, acc);
+}
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// Grid-wide barrier number `epoch` (1, 2, ...).  The last block to arrive runs
+// `last` with all its threads before it releases the others, so the
+// cross-block reductions are done once.  Returns false when the wait ran out
+// (or another block's did); the caller then returns.
+template <typename F>
+__device__ __forceinline__ bool grid_sync(PcgSync *gs, int *error, unsigned long long timeout_ns,
+                                          long long max_polls, unsigned long long epoch,
+                                          F &&last) {
+    __shared__ int s_last, s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned long long old = atomicAdd(&gs->arrive, 1ull);
+        const int lst = old + 1ull == epoch * gridDim.x;
+        if (lst) __threadfence();
+        s_last = lst;
+        s_ok = 1;
+    }
+    __syncthreads();
+    if (s_last) {
+        last();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            st_release(&gs->release, epoch);
+        }
+    } else if (threadIdx.x == 0) {
+        const unsigned long long t0 = global_ns();
+        for (long long poll = 0; ld_acquire(&gs->release) < epoch; ++poll) {
+            if ((poll & 31) == 31 &&
+                (*(volatile int *)error != 0 || poll > max_polls ||
+                 global_ns() - t0 > timeout_ns)) {
+                atomicExch(error, 1);
+                s_ok = 0;
+                break;
+            }
+            __nanosleep(32);
+        }
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+template <typename T>
+struct PcgArgs {
+    const long long *sp;
+    const int *col;
+    const T *val;
+    int n, nslices;
+    long long stored;  // entries of the SELL arrays, padding included
+    const T *B;
+    T *X, *R, *P, *W;
+    int k, max_iter, rel_tol, x_zero;
+    double rate, tol;
+    double matrix_bytes;  // nnz (v + 4) + 4 (n + 1) of S
+    PcgScalars *sc;
+    PcgSync *sync;
+    PcgStats *stats;
+    double *part;  // 2 x gridDim.x x KP
+    // bound of every grid-barrier wait (device clock and poll count)
+    unsigned long long timeout_ns;
+    long long max_polls;
+    // failure-detection test only: the grid's last block returns before its
+    // first barrier, so the others' waits run out (never set otherwise)
+    int withhold_last;
+};
+
+// Compiler-only ordering point between the 16-byte groups of a row in the
+// streaming phases: keeps one group's loads in flight per thread instead of
+// all of them, which bounds the registers (warps supply the parallelism).
+__device__ __forceinline__ void group_fence() { asm volatile("" ::: "memory"); }
+
+__host__ __device__ constexpr int pow2ceil(int x) {
+    int p = 1;
+    while (p < x) p <<= 1;
+    return p;
+}
+
+// Warp sums of N per-lane column values (N a power of two <= 32): returns, in
+// lane l, the sum over the 32 lanes of column l % N.  The first log2(N) steps
+// exchange halves of the values between lanes (a transposing butterfly), the
+// others add single values: N - 1 + log2(32 / N) additions.  FP64 additions
+// occupy a scheduler for 64 clocks each.
+template <typename T, int N>
+__device__ __forceinline__ T warp_cols_reduce(T (&v)[N], int lane) {
+#pragma unroll
+    for (int h = N / 2; h >= 1; h >>= 1) {
+        const bool up = (lane & h) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const T send = up ? v[i] : v[i + h];
+            const T keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+        }
+    }
+    T s = v[0];
+#pragma unroll
+    for (int o = 16; o >= N; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// Adds the warp's column sums of acc[0..KP) to wrow[0..KP) (this warp's row of
+// shared accumulators; lane c owns column c).
+template <typename T, int KP>
+__device__ __forceinline__ void warp_cols_add(const T (&acc)[KP], double *wrow, int lane) {
+    constexpr int K1 = KP < 32 ? KP : 32;
+    constexpr int N1 = pow2ceil(K1);
+    T v[N1];
+#pragma unroll
+    for (int i = 0; i < N1; ++i) v[i] = i < K1 ? acc[i] : T(0);
+    const T s = warp_cols_reduce<T, N1>(v, lane);
+    if (lane < K1) wrow[lane] += (double)s;
+    if constexpr (KP > 32) {
+        constexpr int K2 = KP - 32;
+        constexpr int N2 = pow2ceil(K2);
+        T u[N2];
+#pragma unroll
+        for (int i = 0; i < N2; ++i) u[i] = i < K2 ? acc[32 + i] : T(0);
+        const T s2 = warp_cols_reduce<T, N2>(u, lane);
+        if (lane < K2) wrow[32 + lane] += (double)s2;
+    }
+}
+
+// Column sums of the gridDim.x block partials part[b * KP + c] into
+// out[0..KP) (shared memory), fixed order: thread t adds blocks t / KP,
+// t / KP + S, ... of column t % KP (S = threads / KP stripes), then the
+// stripes are added pairwise in a fixed tree.
+template <int KP, int NT>
+__device__ __forceinline__ void grid_cols_sum(const double *part, double *out, double *stripe) {
+    constexpr int S = NT / KP;
+    const int t = threadIdx.x;
+    if (gridDim.x <= 32) {
+        // few blocks: one thread per column, four chains in a fixed order, no
+        // tree and its barriers
+        if (t < KP) {
+            const int nb = gridDim.x;
+            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+            int b = 0;
+            for (; b + 3 < nb; b += 4) {
+                s0 += __ldcg(part + (size_t)b * KP + t);
+                s1 += __ldcg(part + (size_t)(b + 1) * KP + t);
+                s2 += __ldcg(part + (size_t)(b + 2) * KP + t);
+                s3 += __ldcg(part + (size_t)(b + 3) * KP + t);
+            }
+            for (; b < nb; ++b) s0 += __ldcg(part + (size_t)b * KP + t);
+            out[t] = (s0 + s1) + (s2 + s3);
+        }
+        __syncthreads();
+        return;
+    }
+    double s = 0.0;
+    if (t < S * KP) {
+        const int c = t % KP;
+        const int nb = gridDim.x;
+        int b = t / KP;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        // L2 loads: the partials were written by other blocks on other SMs
+        for (; b + 3 * S < nb; b += 4 * S) {
+            s0 += __ldcg(part + (size_t)b * KP + c);
+            s1 += __ldcg(part + (size_t)(b + S) * KP + c);
+            s2 += __ldcg(part + (size_t)(b + 2 * S) * KP + c);
+            s3 += __ldcg(part + (size_t)(b + 3 * S) * KP + c);
+        }
+        for (; b < nb; b += S) s0 += __ldcg(part + (size_t)b * KP + c);
+        s = (s0 + s1) + (s2 + s3);
+    }
+    stripe[t] = s;
+    __syncthreads();
+    for (int width = S; width > 1;) {
+        const int half = (width + 1) / 2;
+        if (t < (width - half) * KP) stripe[t] += stripe[t + half * KP];
+        __syncthreads();
+        width = half;
+    }
+    if (t < KP) out[t] = stripe[t];
+    __syncthreads();
+}
+
+// Wide blocks (at least 8 column groups, an even number) gather the SpMM
+// phase in two halves of the column groups.
+template <typename T, int KP>
+constexpr bool kSplitGather = (KP / Pk<T>::L) >= 8 && (KP / Pk<T>::L) % 2 == 0;
+
+// Block shape by row width: 512 threads (two resident blocks, <= 64
+// registers) for rows up to 80 bytes and for FP32 rows of 40 columns (whose
+// phases run in two column parts: 4.76 -> 4.34 s of inner solve per 128^3
+// solve against one block per SM), 512 threads (<= 128 registers) up to 160
+// bytes, and 256 threads (<= 255 registers) for wider FP64 rows.
+template <typename T, int KP>
+__host__ __device__ constexpr int pcg_threads() {
+    return sizeof(T) * KP <= 160 ? 512 : 256;
+}
+template <typename T, int KP>
+__host__ __device__ constexpr int pcg_min_blocks() {
+    // FP32 rows of 40 columns fit 64 registers with their phases split into
+    // column parts: two blocks per SM, twice the warps hiding gather latency
+    return (sizeof(T) * KP <= 80 || (sizeof(T) == 4 && KP == 40)) ? 2 : 1;
+}
+
+template <typename T, int KP>
+__global__ void __launch_bounds__(pcg_threads<T, KP>(), pcg_min_blocks<T, KP>())
+k_block_pcg(PcgArgs<T> a) {
+    constexpr int kPcgThreads = pcg_threads<T, KP>();
+    constexpr int L = Pk<T>::L;
+    constexpr int G = KP / L;  // 16-byte groups per row
+    constexpr int nwarps = kPcgThreads / 32;
+    // column-group parts of the setup, SpMM and update phases
+    constexpr int NP = kSplitGather<T, KP> ? 2 : 1;
+    constexpr int GP = G / NP, KPP = KP / NP;
+    auto for_parts = [](auto &&f) {
+        f(std::integral_constant<int, 0>{});
+        if constexpr (NP == 2) f(std::integral_constant<int, 1>{});
+    };
+    __shared__ double wred[nwarps][KP];  // per-warp column sums of one phase
+    __shared__ double stripe[kPcgThreads];
+    __shared__ double sum1[KP], sum2[KP];
+    __shared__ T s_coef[KP];
+    __shared__ int s_act[KP];
+    __shared__ int s_gact[G];
+    __shared__ int s_nactive;
+    __shared__ long long s_range[2];
+
+    PcgScalars *sc = a.sc;
+    PcgSync *gs = a.sync;
+    int *error = &a.sync->error;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int k = a.k, n = a.n;
+    const double vb = (double)sizeof(T);
+    if (a.withhold_last && gridDim.x > 1 && blockIdx.x == gridDim.x - 1) return;
+
+    // per-warp accumulators: clear, and flush (fixed-order sum over warps)
+    auto wred_zero = [&]() {
+        for (int i = tid; i < nwarps * KP; i += kPcgThreads) (&wred[0][0])[i] = 0.0;
+        __syncthreads();
+    };
+    auto wred_flush = [&](double *out) {
+        __syncthreads();
+        if (tid < KP) {
+            double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int w = 0; w < nwarps; ++w) s4[w & 3] += wred[w][tid];
+            out[tid] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        }
+        __syncthreads();
+    };
+
+    // slice range of this block, balanced by stored entries
+    if (tid < 2) {
+        const long long total = a.sp[a.nslices];
+        const long long target = total * (long long)(blockIdx.x + tid) / gridDim.x;
+        int lo = 0, hi = a.nslices;  // first slice s with sp[s] >= target
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (a.sp[mid] < target) lo = mid + 1;
+            else hi = mid;
+        }
+        s_range[tid] = (blockIdx.x + tid == gridDim.x) ? a.nslices : lo;
+    }
+    __syncthreads();
+    const int s0 = (int)s_range[0], s1 = (int)s_range[1];
+    const int r0 = min(n, 32 * s0), r1 = min(n, 32 * s1);
+    unsigned long long epoch = 0;
+    // this block's partial sums, and of a second set (norms of b)
+    double *part1 = a.part + (size_t)blockIdx.x * KP;
+    double *part2 = a.part + (size_t)(gridDim.x + blockIdx.x) * KP;
+
+    auto finish = [&](bool ok) {
+        if (blockIdx.x == 0 && tid == 0) {
+            if (!ok || *(volatile int *)error) a.stats->error = 1;
+            a.stats->launches += 1;
+            a.stats->iters += (unsigned long long)sc->niter;
+        }
+    };
+
+    // ---------------- r = b - S x (or r = b for x = 0), p = 0, norms
+    // (wide blocks work on their column groups in parts, which bounds the
+    // accumulator registers of every phase)
+    wred_zero();
+    if (a.x_zero) {
+        for_parts([&](auto part) {
+            constexpr int U0 = decltype(part)::value * GP;
+            T racc[KPP];
+#pragma unroll
+            for (int c = 0; c < KPP; ++c) racc[c] = T(0);
+            for (int row = r0 + tid; row < r1; row += kPcgThreads) {
+#pragma unroll
+                for (int uu = 0; uu < GP; ++uu) {
+                    const int u = U0 + uu;
+                    const Pk<T> b = Pk<T>::ld(a.B + boff<T, KP>(row, u));
+                    Pk<T> z;
+#pragma unroll
+                    for (int q = 0; q < L; ++q) {
+                        z.v[q] = T(0);
+                        racc[uu * L + q] = fma(b.v[q], b.v[q], racc[uu * L + q]);
+                    }
+                    b.st(a.R + boff<T, KP>(row, u));
+                    z.st(a.X + boff<T, KP>(row, u));
+                    z.st(a.P + boff<T, KP>(row, u));
+                    group_fence();
+                }
+            }
+            warp_cols_add<T, KPP>(racc, wred[warp] + U0 * L, lane);
+        });
+    } else {
+        for (int s = s0 + warp; s < s1; s += nwarps) {
+            const long long beg = a.sp[s], end = a.sp[s + 1];
+            const int row = s * 32 + lane;
+            for_parts([&](auto part) {
+                constexpr int U0 = decltype(part)::value * GP;
+                T acc[KPP];
+#pragma unroll
+                for (int c = 0; c < KPP; ++c) acc[c] = T(0);
+                gather_row_part<T, KP, U0, GP>(a.col, a.val, beg + lane, (int)((end - beg) >> 5),
+                                               a.X, acc);
+                if (row < n) {
+#pragma unroll
+                    for (int uu = 0; uu < GP; ++uu) {
+                        const int u = U0 + uu;
+                        const Pk<T> b = Pk<T>::ld(a.B + boff<T, KP>(row, u));
+                        Pk<T> r, z;
+#pragma unroll
+                        for (int q = 0; q < L; ++q) {
+                            r.v[q] = b.v[q] - acc[uu * L + q];
+                            z.v[q] = T(0);
+                            acc[uu * L + q] = r.v[q] * r.v[q];
+                        }
+                        r.st(a.R + boff<T, KP>(row, u));
+                        z.st(a.P + boff<T, KP>(row, u));
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < KPP; ++c) acc[c] = T(0);
+                }
+                warp_cols_add<T, KPP>(acc, wred[warp] + U0 * L, lane);
+            });
+        }
+    }
+    wred_flush(part1);
+    if (a.rel_tol) {
+        wred_zero();
+        for_parts([&](auto part) {
+            constexpr int U0 = decltype(part)::value * GP;
+            T bacc[KPP];
+#pragma unroll
+            for (int c = 0; c < KPP; ++c) bacc[c] = T(0);
+            for (int row = r0 + tid; row < r1; row += kPcgThreads) {
+#pragma unroll
+                for (int uu = 0; uu < GP; ++uu) {
+                    const Pk<T> b = Pk<T>::ld(a.B + boff<T, KP>(row, U0 + uu));
+#pragma unroll
+                    for (int q = 0; q < L; ++q)
+                        bacc[uu * L + q] = fma(b.v[q], b.v[q], bacc[uu * L + q]);
+                    group_fence();
+                }
+            }
+            warp_cols_add<T, KPP>(bacc, wred[warp] + U0 * L, lane);
+        });
+        wred_flush(part2);
+    }
+    // initial residual norms (src/ops_lin_sol.c:171-233)
+    if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
+            grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
+            if (a.rel_tol)
+                grid_cols_sum<KP, kPcgThreads>(a.part + (size_t)gridDim.x * KP, sum2, stripe);
+            if (tid < kPcgMaxCols) {
+                const int c = tid;
+                if (c < k) {
+                    const double nb = a.rel_tol ? sqrt(sum2[c]) : 1.0;
+                    const double rr = sum1[c];
+                    sc->norm_b[c] = nb;
+                    sc->rho2[c] = rr;
+                    sc->init_res[c] = sqrt(rr);
+                    sc->last_res[c] = sqrt(rr);
+                    sc->active[c] = sqrt(rr) > a.tol * nb ? 1 : 0;
+                    sc->left_at[c] = 0;
+                    sc->beta[c] = 0.0;
+                    sc->alpha[c] = 0.0;
+                } else {
+                    sc->active[c] = 0;
+                    sc->left_at[c] = 0;
+                }
+            }
+            __syncthreads();
+            if (tid == 0) {
+                int cnt = 0;
+                for (int c = 0; c < k; ++c) cnt += sc->active[c];
+                sc->nactive = cnt;
+                sc->niter = 0;
+                a.stats->kernel_bytes +=
+                    a.x_zero ? 4.0 * n * KP * vb : a.matrix_bytes + 4.0 * n * KP * vb;
+            }
+        })) {
+        finish(false);
+        return;
+    }
+
+    for (int it = 0; it < a.max_iter; ++it) {
+        // ---------------- phase 1: p = r + beta p
+        if (tid < KP) {
+            s_act[tid] = sc->active[tid];
+            s_coef[tid] = (T)sc->beta[tid];
+        }
+        if (tid == 0) s_nactive = sc->nactive;
+        __syncthreads();
+        if (s_nactive == 0) break;
+        if (tid < G) {
+            int any = 0;
+            for (int q = 0; q < L; ++q) any |= s_act[tid * L + q];
+            s_gact[tid] = any;
+        }
+        __syncthreads();
+        const bool first = it == 0;
+        for (int row = r0 + tid; row < r1; row += kPcgThreads) {
+#pragma unroll
+            for (int u = 0; u < G; ++u) {
+                if (!s_gact[u]) continue;
+                const Pk<T> r = Pk<T>::ld(a.R + boff<T, KP>(row, u));
+                Pk<T> p = Pk<T>::ld(a.P + boff<T, KP>(row, u));
+#pragma unroll
+                for (int q = 0; q < L; ++q)
+                    if (s_act[u * L + q])
+                        p.v[q] = first ? r.v[q] : fma(s_coef[u * L + q], p.v[q], r.v[q]);
+                p.st(a.P + boff<T, KP>(row, u));
+                group_fence();
+            }
+        }
+        wred_zero();
+        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
+                if (tid == 0) a.sync->t_spmm = global_ns();
+            })) {
+            finish(false);
+            return;
+        }
+
+        // ---------------- phase 2: w = S p, p^T w
+        {
+            bool ga[G];
+#pragma unroll
+            for (int u = 0; u < G; ++u) ga[u] = s_gact[u] != 0;
+            for (int s = s0 + warp; s < s1; s += nwarps) {
+                const long long beg = a.sp[s], end = a.sp[s + 1];
+                const int width = (int)((end - beg) >> 5);
+                if constexpr (kSplitGather<T, KP>) {
+                    // one half of the column groups of a slice's rows: w, then the
+                    // partial sums of p^T w over those columns
+                    auto spmm_half = [&](auto half_tag, int s, int width, long long e0) {
+                        constexpr int H = decltype(half_tag)::value;
+                        constexpr int NU = G / 2, U0 = H * NU;
+                        T acc[NU * L];
+#pragma unroll
+                        for (int c = 0; c < NU * L; ++c) acc[c] = T(0);
+                        gather_row_part<T, KP, U0, NU>(a.col, a.val, e0, width, a.P, acc);
+                        const int row = s * 32 + lane;
+#pragma unroll
+                        for (int u = 0; u < NU; ++u) {
+                            if (!ga[U0 + u] || row >= n) {
+#pragma unroll
+                                for (int q = 0; q < L; ++q) acc[u * L + q] = T(0);
+                                continue;
+                            }
+                            Pk<T> w;
+#pragma unroll
+                            for (int q = 0; q < L; ++q) w.v[q] = acc[u * L + q];
+                            w.st(a.W + boff<T, KP>(row, U0 + u));
+                            const Pk<T> p = Pk<T>::ld(a.P + boff<T, KP>(row, U0 + u));
+#pragma unroll
+                            for (int q = 0; q < L; ++q)
+                                acc[u * L + q] = s_act[(U0 + u) * L + q] ? p.v[q] * w.v[q] : T(0);
+                        }
+                        warp_cols_add<T, NU * L>(acc, wred[warp] + U0 * L, lane);
+                    };
+                    spmm_half(std::integral_constant<int, 0>{}, s, width, beg + lane);
+                    spmm_half(std::integral_constant<int, 1>{}, s, width, beg + lane);
+                } else {
+                    T acc[KP];
+#pragma unroll
+                    for (int c = 0; c < KP; ++c) acc[c] = T(0);
+                    gather_row<T, KP>(a.col, a.val, beg + lane, width, a.P, ga, acc);
+                    const int row = s * 32 + lane;
+                    if (row < n) {
+#pragma unroll
+                        for (int u = 0; u < G; ++u) {
+                            if (!ga[u]) continue;
+                            Pk<T> w;
+#pragma unroll
+                            for (int q = 0; q < L; ++q) w.v[q] = acc[u * L + q];
+                            w.st(a.W + boff<T, KP>(row, u));
+                            const Pk<T> p = Pk<T>::ld(a.P + boff<T, KP>(row, u));
+#pragma unroll
+                            for (int q = 0; q < L; ++q)
+                                acc[u * L + q] = s_act[u * L + q] ? p.v[q] * w.v[q] : T(0);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < KP; ++c) acc[c] = T(0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < G; ++u)
+                        if (!ga[u]) {
+#pragma unroll
+                            for (int q = 0; q < L; ++q) acc[u * L + q] = T(0);
+                        }
+                    warp_cols_add<T, KP>(acc, wred[warp], lane);
+                }
+            }
+            wred_flush(part1);
+        }
+        // alpha = rho / p^T w (src/ops_lin_sol.c:300-330)
+        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
+                grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
+                if (tid < k) {
+                    const int c = tid;
+                    const double ptw = sum1[c];
+                    sc->ptw[c] = ptw;
+                    sc->rho1[c] = sc->rho2[c];
+                    sc->alpha[c] = sc->active[c] ? sc->rho2[c] / ptw : 0.0;
+                }
+                if (tid == 0) {
+                    int gact = 0;
+                    for (int u = 0; u < G; ++u) gact += s_gact[u];
+                    const double vec = (double)n * gact * L * vb;
+                    a.stats->spmm_ns += global_ns() - a.sync->t_spmm;
+                    // SpMM: the matrix once, p read once, w written once
+                    a.stats->spmm_bytes += a.matrix_bytes + 2.0 * vec;
+                    // iteration: phase 1 (r, p read; p written), phase 2 (p
+                    // gathered and re-read, w written), phase 3 (x, p, r, w
+                    // read; x, r written)
+                    a.stats->kernel_bytes += a.matrix_bytes + 12.0 * vec;
+                }
+            })) {
+            finish(false);
+            return;
+        }
+
+        // ---------------- phase 3: x += alpha p, r -= alpha w, r^T r
+        if (tid < KP) s_coef[tid] = (T)sc->alpha[tid];
+        wred_zero();
+        for_parts([&](auto part) {
+            constexpr int U0 = decltype(part)::value * GP;
+            T racc[KPP];
+#pragma unroll
+            for (int c = 0; c < KPP; ++c) racc[c] = T(0);
+            for (int row = r0 + tid; row < r1; row += kPcgThreads) {
+#pragma unroll
+                for (int uu = 0; uu < GP; ++uu) {
+                    const int u = U0 + uu;
+                    if (!s_gact[u]) continue;
+                    Pk<T> x = Pk<T>::ld(a.X + boff<T, KP>(row, u));
+                    Pk<T> r = Pk<T>::ld(a.R + boff<T, KP>(row, u));
+                    const Pk<T> p = Pk<T>::ld(a.P + boff<T, KP>(row, u));
+                    const Pk<T> w = Pk<T>::ld(a.W + boff<T, KP>(row, u));
+#pragma unroll
+                    for (int q = 0; q < L; ++q) {
+                        const int c = u * L + q;
+                        if (s_act[c]) {
+                            const T al = s_coef[c];
+                            x.v[q] = fma(al, p.v[q], x.v[q]);
+                            r.v[q] = fma(-al, w.v[q], r.v[q]);
+                            racc[uu * L + q] = fma(r.v[q], r.v[q], racc[uu * L + q]);
+                        }
+                    }
+                    x.st(a.X + boff<T, KP>(row, u));
+                    r.st(a.R + boff<T, KP>(row, u));
+                    group_fence();
+                }
+            }
+            warp_cols_add<T, KPP>(racc, wred[warp] + U0 * L, lane);
+        });
+        wred_flush(part1);
+        // convergence test of src/ops_lin_sol.c:383-394 and beta for the next step
+        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
+                grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
+                if (tid < k && sc->active[tid]) {
+                    const int c = tid;
+                    const double rr = sum1[c];
+                    sc->rho2[c] = rr;
+                    const double res = sqrt(rr);
+                    sc->last_res[c] = res;
+                    sc->beta[c] = rr / sc->rho1[c];
+                    if (!(res > a.rate * sc->init_res[c] && res > a.tol * sc->norm_b[c])) {
+                        sc->active[c] = 0;
+                        sc->left_at[c] = sc->niter + 1;  // niter moves on after the barrier
+                    }
+                }
+                __syncthreads();
+                if (tid == 0) {
+                    int cnt = 0;
+                    for (int c = 0; c < k; ++c) cnt += sc->active[c];
+                    sc->nactive = cnt;
+                    sc->niter += 1;
+                }
+            })) {
+            finish(false);
+            return;
+        }
+    }
+    finish(true);
+}
+
+// ---------------------------------------------------------------- small operators
+// Grid-wide barrier number `epoch` without a last block's turn: every block
+// waits for the arrivals of all.  Bounded as grid_sync is.
+__device__ __forceinline__ bool grid_arrive_wait(PcgSync *gs, int *error,
+                                                 unsigned long long timeout_ns,
+                                                 long long max_polls, unsigned long long epoch) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_ok = 1;
+        __threadfence();
+        const unsigned long long all = epoch * gridDim.x;
+        if (atomicAdd(&gs->arrive, 1ull) + 1ull < all) {
+            const unsigned long long t0 = global_ns();
+            for (long long poll = 0; ld_acquire(&gs->arrive) < all; ++poll) {
+                if ((poll & 31) == 31 &&
+                    (*(volatile int *)error != 0 || poll > max_polls ||
+                     global_ns() - t0 > timeout_ns)) {
+                    atomicExch(error, 1);
+                    s_ok = 0;
+                    break;
+                }
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// The same block CG for operators whose step is a chain of latencies rather
+// than bytes or FMAs: phases of a microsecond between barriers.
+//
+// Work unit: one slice (32 rows, a row per lane) times one chunk of GU (one or
+// two) 16-byte column groups, so that a narrow operator still fills the warps
+// (an FP64 FMA occupies a scheduler for 64 clocks: 20 FP64 columns in one warp
+// per slice took 42 us a step at n = 4160).  A warp keeps its U units for the
+// whole solve with their x, r, p and w in registers; global memory holds only
+// what other units gather.  Every block sums the partials of all blocks itself
+// and keeps its own scalars, in shared memory, as are the block's matrix
+// entries where they fit.
+//
+// FUSE (two phases, two barriers a step): a gather forms p = r + beta p of each
+// neighbour as it reads r and p, and the own rows' p is stored with r after the
+// alpha barrier.  Otherwise (FP64 operators with enough entries per row that
+// the gather's second FMA costs more than a barrier): p is stored first, and
+// gathered after a barrier of its own.  CL: the blocks are one thread-block
+// cluster and its hardware barrier replaces the grid's.
+//
+constexpr int kSmallThreads = 512;
+constexpr int kSmallSmemMax = 160 * 1024;  // the rest stays L1
+// Element offset of row i, 16-byte group u of a slice-blocked block of G groups
+// (a small operator's blocks have fewer than 2^31 elements).
+template <typename T>
+__device__ __forceinline__ unsigned goff(int i, int u, int G) {
+    constexpr unsigned L = Pk<T>::L;
+    return (((unsigned)i >> 5) * (unsigned)G + (unsigned)u) * (32u * L) + ((unsigned)i & 31u) * L;
+}
+
+// acc += N entries (col[0], col[32], ..) of the lane's row times the groups
+// [u0, u0 + GU) of V, or with RP of V + beta Vp.  A group past the last one
+// repeats it; its sums are not used.
+template <typename T, int GU, int N, bool RP>
+__device__ __forceinline__ void unit_entries(const int *col, const T *val, const T *V, const T *Vp,
+                                             const T *beta, int u0, int G,
+                                             T (&acc)[GU * Pk<T>::L]) {
+    constexpr int L = Pk<T>::L;
+    int j[N];
+    T m[N];
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+        j[d] = col[32 * d];
+        m[d] = val[32 * d];
+    }
+    Pk<T> q0[N][GU], q1[N][GU];
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+#pragma unroll
+        for (int g = 0; g < GU; ++g) {
+            const unsigned o = goff<T>(j[d], g == 0 ? u0 : min(u0 + g, G - 1), G);
+            q0[d][g] = Pk<T>::ld(V + o);
+            if constexpr (RP) q1[d][g] = Pk<T>::ld(Vp + o);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < N; ++d) {
+#pragma unroll
+        for (int g = 0; g < GU; ++g) {
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                T y = q0[d][g].v[l];
+                if constexpr (RP) y = fma(beta[g * L + l], q1[d][g].v[l], y);
+                acc[g * L + l] = fma(m[d], y, acc[g * L + l]);
+            }
+        }
+    }
+}
+template <typename T, int GU, int NE, bool RP>
+__device__ __forceinline__ void unit_gather(const int *col, const T *val, int width, const T *V,
+                                            const T *Vp, const T *sbeta, int u0, int G,
+                                            T (&acc)[GU * Pk<T>::L]) {
+    constexpr int CC = GU * Pk<T>::L;
+    T beta[CC];
+#pragma unroll
+    for (int c = 0; c < CC; ++c) {
+        acc[c] = T(0);
+        beta[c] = RP ? sbeta[c] : T(0);
+    }
+    int e = 0;
+#pragma unroll 1
+    for (; e + NE <= width; e += NE)
+        unit_entries<T, GU, NE, RP>(col + 32 * e, val + 32 * e, V, Vp, beta, u0, G, acc);
+#pragma unroll 1
+    for (; e < width; ++e)
+        unit_entries<T, GU, 1, RP>(col + 32 * e, val + 32 * e, V, Vp, beta, u0, G, acc);
+}
+
+template <typename T, int GU, int U, bool CL, bool FUSE>
+__global__ void __launch_bounds__(kSmallThreads, 1)
+k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
+    constexpr int L = Pk<T>::L, CC = GU * L;
+    constexpr int NW = kSmallThreads / 32;
+    constexpr int NE = 8 / (U * GU * (FUSE ? 2 : 1));  // matrix entries in flight per lane
+    extern __shared__ __align__(16) unsigned char dsm[];
+    __shared__ double wred[NW * U][CC];  // column sums of each unit
+    __shared__ double sums[2][kPcgMaxCols];
+    __shared__ double stripe[kSmallThreads];
+    __shared__ T s_alpha[kPcgMaxCols], s_beta[kPcgMaxCols];
+    __shared__ int s_act[kPcgMaxCols];
+    __shared__ int s_nactive;
+    __shared__ PcgScalars s_sc;
+    PcgScalars *sc = &s_sc;
+    PcgSync *gs = a.sync;
+    int *error = &a.sync->error;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int k = a.k, n = a.n, G = kp / L, nch = (G + GU - 1) / GU;
+    const int nb = gridDim.x, me = blockIdx.x;
+    const bool stats_block = me == 0;
+    if (!CL && a.withhold_last && nb > 1 && me == nb - 1) return;
+
+    const int s0 = (int)((long long)a.nslices * me / nb);
+    const int s1 = (int)((long long)a.nslices * (me + 1) / nb);
+    const int nsl = s1 - s0;  // nsl nch <= U NW by the launch's choice
+    // the block's matrix entries in shared memory where they fit
+    const long long e_lo = a.sp[s0], e_cnt = a.sp[s1] - e_lo;
+    const bool in_smem = e_cnt * (long long)(sizeof(T) + 4) <= smem_bytes;
+    T *sval = reinterpret_cast<T *>(dsm);
+    int *scol = reinterpret_cast<int *>(sval + (in_smem ? e_cnt : 0));
+    if (in_smem) {
+        for (int i = tid; i < (int)e_cnt; i += kSmallThreads) {
+            sval[i] = a.val[e_lo + i];
+            scol[i] = a.col[e_lo + i];
+        }
+    }
+    for (int c = tid; c < kPcgMaxCols; c += kSmallThreads) {
+        s_act[c] = 0;
+        s_alpha[c] = s_beta[c] = T(0);
+    }
+    __syncthreads();
+
+    // this warp's units
+    int slice[U], u0[U], width[U], ent[U];
+    bool live[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        const int v = warp + i * NW;
+        live[i] = v < nsl * nch;
+        slice[i] = live[i] ? s0 + v / nch : s0;
+        u0[i] = live[i] ? (v % nch) * GU : 0;
+        const long long beg = live[i] ? a.sp[slice[i]] : 0, end = live[i] ? a.sp[slice[i] + 1] : 0;
+        width[i] = (int)((end - beg) >> 5);
+        ent[i] = (int)(beg - e_lo) + lane;
+    }
+    auto has_row = [&](int i) { return slice[i] * 32 + lane < n; };
+    T x[U][CC], r[U][CC], p[U][CC], w[U][CC];
+
+    // w = the unit's rows of S V, and of S (R + beta P)
+    auto gather = [&](int i, const T *V, T (&acc)[CC]) {
+        if (in_smem)
+            unit_gather<T, GU, NE, false>(scol + ent[i], sval + ent[i], width[i], V, V, s_beta, u0[i],
+                                      G, acc);
+        else
+            unit_gather<T, GU, NE, false>(a.col + e_lo + ent[i], a.val + e_lo + ent[i], width[i], V, V,
+                                      s_beta, u0[i], G, acc);
+    };
+    auto gather_rp = [&](int i, T (&acc)[CC]) {
+        if (in_smem)
+            unit_gather<T, GU, NE, true>(scol + ent[i], sval + ent[i], width[i], a.R, a.P,
+                                     s_beta + u0[i] * L, u0[i], G, acc);
+        else
+            unit_gather<T, GU, NE, true>(a.col + e_lo + ent[i], a.val + e_lo + ent[i], width[i], a.R,
+                                     a.P, s_beta + u0[i] * L, u0[i], G, acc);
+    };
+    auto store = [&](T *v, int i, const T (&q)[CC]) {
+#pragma unroll
+        for (int g = 0; g < GU; ++g)
+            if (u0[i] + g < G && has_row(i)) {
+                Pk<T> o;
+#pragma unroll
+                for (int l = 0; l < L; ++l) o.v[l] = q[g * L + l];
+                o.st(v + goff<T>(slice[i] * 32 + lane, u0[i] + g, G));
+            }
+    };
+    auto load = [&](const T *v, int i, T (&q)[CC]) {
+#pragma unroll
+        for (int g = 0; g < GU; ++g) {
+            const bool in = live[i] && u0[i] + g < G && has_row(i);
+            Pk<T> o;
+            if (in) o = Pk<T>::ld(v + goff<T>(slice[i] * 32 + lane, u0[i] + g, G));
+#pragma unroll
+            for (int l = 0; l < L; ++l) q[g * L + l] = in ? o.v[l] : T(0);
+        }
+    };
+    // column sums of q over the unit's rows, into its row of wred
+    auto unit_sum = [&](int i, T (&q)[CC]) {
+        const T s = warp_cols_reduce<T, CC>(q, lane);
+        if (lane < CC) wred[warp + i * NW][lane] = (double)s;
+    };
+    // Two sets of partials alternate by the barrier's parity: blocks read them
+    // after a barrier while faster ones already write the next phase's, and a set
+    // is rewritten only after the following barrier.
+    unsigned long long epoch = 0;
+    auto part_of = [&](unsigned long long e, int which) {
+        return a.part + ((size_t)(e & 1) * 2 + which) * nb * kp;
+    };
+    // this block's column sums of wred, for the next barrier
+    auto publish = [&](int which) {
+        __syncthreads();
+        if (tid < kp) {
+            const int ch = tid / CC, c = tid % CC;
+            double s4[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int sl = 0; sl < nsl; ++sl) s4[sl & 3] += wred[sl * nch + ch][c];
+            part_of(epoch + 1, which)[(size_t)me * kp + tid] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+        }
+    };
+    // Sums of the partials over the blocks: `stripes` threads per column, each
+    // a fixed share of the blocks, then a fixed tree.
+    auto total = [&](int which, double *out) {
+        const double *part = part_of(epoch, which);
+        const int stripes = kSmallThreads / kp;
+        const int c = tid % kp, st = tid / kp;
+        double t0 = 0.0, t1 = 0.0;
+        if (st < stripes) {
+            int b = st;
+            for (; b + stripes < nb; b += 2 * stripes) {
+                t0 += __ldcg(part + (size_t)b * kp + c);
+                t1 += __ldcg(part + (size_t)(b + stripes) * kp + c);
+            }
+            if (b < nb) t0 += __ldcg(part + (size_t)b * kp + c);
+        }
+        stripe[tid] = t0 + t1;
+        __syncthreads();
+        for (int wd = min(stripes, nb); wd > 1;) {
+            const int half = (wd + 1) / 2;
+            if (tid < (wd - half) * kp) stripe[tid] += stripe[tid + half * kp];
+            __syncthreads();
+            wd = half;
+        }
+        if (tid < kp) out[tid] = stripe[tid];
+        __syncthreads();
+    };
+    auto barrier = [&]() {
+        ++epoch;
+        if constexpr (CL) {
+            cooperative_groups::this_cluster().sync();
+            return true;
+        } else {
+            return grid_arrive_wait(gs, error, a.timeout_ns, a.max_polls, epoch);
+        }
+    };
+    auto finish = [&](bool ok) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+            if (live[i]) store(a.X, i, x[i]);
+        if (me == 0) {  // the host reads the first block's scalars
+            const int *src = reinterpret_cast<const int *>(sc);
+            int *dst = reinterpret_cast<int *>(a.sc);
+            for (int i = tid; i < (int)(sizeof(PcgScalars) / sizeof(int)); i += kSmallThreads)
+                dst[i] = src[i];
+        }
+        if (me == 0 && tid == 0) {
+            if (!ok || *(volatile int *)error) a.stats->error = 1;
+            a.stats->launches += 1;
+            a.stats->iters += (unsigned long long)sc->niter;
+        }
+    };
+
+    // ---------------- r = b - S x (or r = b for x = 0), p = 0, norms
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        T b[CC], q[CC];
+        load(a.B, i, b);
+        if (a.x_zero) {
+#pragma unroll
+            for (int c = 0; c < CC; ++c) x[i][c] = w[i][c] = T(0);
+        } else {
+            load(a.X, i, x[i]);
+            if (live[i]) gather(i, a.X, w[i]);
+        }
+#pragma unroll
+        for (int c = 0; c < CC; ++c) {
+            p[i][c] = T(0);
+            r[i][c] = live[i] && has_row(i) ? (a.x_zero ? b[c] : b[c] - w[i][c]) : T(0);
+            q[c] = r[i][c] * r[i][c];
+        }
+        if (live[i]) {
+            if constexpr (FUSE) {
+                store(a.R, i, r[i]);
+                store(a.P, i, p[i]);
+            }
+            unit_sum(i, q);
+        }
+    }
+    publish(0);
+    if (a.rel_tol) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            T b[CC];
+            load(a.B, i, b);
+#pragma unroll
+            for (int c = 0; c < CC; ++c) b[c] = b[c] * b[c];
+            if (live[i]) unit_sum(i, b);
+        }
+        publish(1);
+    }
+    if (!barrier()) {
+        if (tid == 0) sc->niter = 0;
+        finish(false);
+        return;
+    }
+    // initial residual norms (src/ops_lin_sol.c:171-233)
+    total(0, sums[0]);
+    if (a.rel_tol) total(1, sums[1]);
+    if (tid < kPcgMaxCols) {
+        const int c = tid;
+        int on = 0;
+        if (c < k) {
+            const double nrm = a.rel_tol ? sqrt(sums[1][c]) : 1.0;
+            const double rr = sums[0][c], res = sqrt(rr);
+            sc->norm_b[c] = nrm;
+            sc->rho2[c] = rr;
+            sc->init_res[c] = res;
+            sc->last_res[c] = res;
+            sc->beta[c] = 0.0;
+            sc->alpha[c] = 0.0;
+            on = res > a.tol * nrm ? 1 : 0;
+        }
+        sc->active[c] = s_act[c] = on;
+        sc->left_at[c] = 0;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int cnt = 0;
+        for (int c = 0; c < k; ++c) cnt += s_act[c];
+        s_nactive = sc->nactive = cnt;
+        sc->niter = 0;
+        if (stats_block)
+            a.stats->kernel_bytes += (a.x_zero ? 0.0 : a.matrix_bytes) + 4.0 * n * kp * sizeof(T);
+    }
+    __syncthreads();
+
+    for (int it = 0; it < a.max_iter && s_nactive > 0; ++it) {
+        // units none of whose columns is active rest
+        bool act[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            int any = 0;
+#pragma unroll
+            for (int c = 0; c < CC; ++c) any |= s_act[u0[i] * L + c];
+            act[i] = live[i] && any != 0;
+        }
+        // ---------------- p = r + beta p
+#pragma unroll
+        for (int i = 0; i < U; ++i)
+            if (act[i]) {
+#pragma unroll
+                for (int c = 0; c < CC; ++c)
+                    if (s_act[u0[i] * L + c]) p[i][c] = fma(s_beta[u0[i] * L + c], p[i][c], r[i][c]);
+                if constexpr (!FUSE) store(a.P, i, p[i]);
+            }
+        if constexpr (!FUSE) {
+            if (!barrier()) {
+                finish(false);
+                return;
+            }
+        }
+        if (tid == 0 && stats_block) gs->t_spmm = global_ns();
+        // ---------------- w = S p, p^T w
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            T q[CC];
+#pragma unroll
+            for (int c = 0; c < CC; ++c) q[c] = T(0);
+            if (act[i]) {
+                if constexpr (FUSE) gather_rp(i, w[i]);
+                else gather(i, a.P, w[i]);
+#pragma unroll
+                for (int c = 0; c < CC; ++c)
+                    q[c] = s_act[u0[i] * L + c] && has_row(i) ? p[i][c] * w[i][c] : T(0);
+            }
+            if (live[i]) unit_sum(i, q);
+        }
+        publish(0);
+        if (!barrier()) {
+            finish(false);
+            return;
+        }
+        // alpha = rho / p^T w (src/ops_lin_sol.c:300-330)
+        total(0, sums[0]);
+        if (tid < k) {
+            const int c = tid;
+            const double ptw = sums[0][c], rho = sc->rho2[c];
+            const double al = s_act[c] ? rho / ptw : 0.0;
+            sc->ptw[c] = ptw;
+            sc->rho1[c] = rho;
+            sc->alpha[c] = al;
+            s_alpha[c] = (T)al;
+        }
+        if (tid == 32 && stats_block) {
+            int gact = 0;
+            for (int u = 0; u < G; ++u) {
+                int any = 0;
+                for (int l = 0; l < L; ++l) any |= s_act[u * L + l];
+                gact += any != 0;
+            }
+            const double vec = (double)n * gact * L * sizeof(T);
+            a.stats->spmm_ns += global_ns() - gs->t_spmm;
+            a.stats->spmm_bytes += a.matrix_bytes + 2.0 * vec;
+            a.stats->kernel_bytes += a.matrix_bytes + 12.0 * vec;
+        }
+        __syncthreads();
+        // ---------------- x += alpha p, r -= alpha w, r^T r
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            T q[CC];
+#pragma unroll
+            for (int c = 0; c < CC; ++c) {
+                q[c] = T(0);
+                if (act[i] && s_act[u0[i] * L + c]) {
+                    const T al = s_alpha[u0[i] * L + c];
+                    x[i][c] = fma(al, p[i][c], x[i][c]);
+                    r[i][c] = fma(-al, w[i][c], r[i][c]);
+                    q[c] = has_row(i) ? r[i][c] * r[i][c] : T(0);
+                }
+            }
+            if constexpr (FUSE) {
+                if (act[i]) {
+                    store(a.R, i, r[i]);
+                    store(a.P, i, p[i]);
+                }
+            }
+            if (live[i]) unit_sum(i, q);
+        }
+        publish(0);
+        if (!barrier()) {
+            finish(false);
+            return;
+        }
+        // convergence test of src/ops_lin_sol.c:383-394 (threads 64 on) and beta
+        // for the next step
+        total(0, sums[0]);
+        if (tid < k && s_act[tid]) {
+            const double rr = sums[0][tid], be = rr / sc->rho1[tid];
+            sc->rho2[tid] = rr;
+            sc->beta[tid] = be;
+            s_beta[tid] = (T)be;
+        }
+        int leave = 0;
+        if (tid >= 64 && tid < 64 + k && s_act[tid - 64]) {
+            const int c = tid - 64;
+            const double res = sqrt(sums[0][c]);
+            sc->last_res[c] = res;
+            if (!(res > a.rate * sc->init_res[c] && res > a.tol * sc->norm_b[c])) {
+                sc->active[c] = 0;
+                sc->left_at[c] = it + 1;
+                leave = 1;
+            }
+        }
+        const int left = __syncthreads_count(leave);
+        if (leave) s_act[tid - 64] = 0;
+        if (tid == 0) {
+            s_nactive -= left;
+            sc->nactive = s_nactive;
+            sc->niter = it + 1;
+        }
+        __syncthreads();
+    }
+    finish(true);
+}
+
+// Cluster size the cluster form may have (16 CTAs where the device schedules
+// such a cluster, else 8), or 0 when neither can run.
+template <typename T, int GU, int U>
+int pcg_small_cluster() {
+    static PerDevice<int> cache;
+    return cache.get([] {
+        auto *kern = k_pcg_small<T, GU, U, true, true>;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kSmallSmemMax) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        for (int c : {16, 8}) {
+            if (c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                              1) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
+            }
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(c);
+            cfg.blockDim = dim3(kSmallThreads);
+            cfg.dynamicSmemBytes = kSmallSmemMax;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = c;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int nc = 0;
+            if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
+            }
+            if (nc > 0) return c;
+        }
+        return 0;
+    });
+}
+
+template <typename T, int GU, int U, bool FUSE>
+void launch_pcg_small_form(const PcgArgs<T> &a, int kp, bool cluster, int nb, cudaStream_t st) {
+    // room for a block's matrix entries, a quarter more than an even share; a
+    // block with more reads them from global memory
+    const double share = 1.25 * (double)a.stored / nb * (sizeof(T) + 4.0) + 4096.0;
+    const int smem = (int)std::min((double)kSmallSmemMax, share) & ~15;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nb);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (FUSE && cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = nb;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_small<T, GU, U, true, true>, a, kp, smem));
+    } else {
+        static PerDevice<bool> smem_set;
+        smem_set.get([] {
+            GCGE_CUDA(cudaFuncSetAttribute(k_pcg_small<T, GU, U, false, FUSE>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kSmallSmemMax));
+            return true;
+        });
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_small<T, GU, U, false, FUSE>, a, kp, smem));
+    }
+    count_launch();
+}
+
+// Runs the solve in k_pcg_small where the units of its operator fit the warps
+// (two each); false where they do not, and the three-phase grid kernel takes it.
+// Measured, us per step, three-phase kernel (or its former cluster form) ->
+// this one:
+//   5-point n = 4160    k = 4 FP32 9.3 -> 7.7, FP64 16 -> 11.8; k = 20 FP64 37 -> 13.6
+//   5-point n = 16384   k = 4 FP32 13 -> 10.7, FP64 24 -> 12.4; k = 20 27 -> 12.8, 38 -> 22.8
+//   7-point 32^3        k = 4 FP32 22 -> 11.8, FP64 26 -> 15.4; k = 20 FP32 29 -> 17.0
+//   27-point 24^3       k = 20 FP32 36 -> 15.1, FP64 59 -> 29.5; 40^3 k = 12 FP32 32 -> 22.5
+// FUSE: the gather's second vector against a barrier.  In FP64 its FMAs decide
+// (entries k / 2 clocks over the SMs; 5-point k = 20, n = 7400: 16.8 us both at
+// 2429, k = 12 14.1 against 14.8 at 1458, k = 40 26.2 against 24.5 at 4859), in
+// FP32 its loads (27-point 24^3, k = 20 15.1 against 15.3 at 23900, k = 40 20.0
+// against 18.4 at 47700).
+// Cluster or grid: the cluster's barriers are shorter, but it has 16 of the 152
+// SMs (FP32 n = 4160: k = 4 7.7 against 10.5 us, k = 12 10.5 against 11.1, k = 20
+// 11.9 against 11.6; FP64 k = 4 11.8 both).
+template <typename T>
+constexpr double kFuseClocks = sizeof(T) == 8 ? 2200.0 : 30000.0;
+template <typename T>
+constexpr double kClusterClocks = sizeof(T) == 8 ? 6000.0 : 2000.0;
+template <typename T>
+bool launch_pcg_small(const PcgArgs<T> &a, int kp, cudaStream_t st) {
+    constexpr int NW = kSmallThreads / 32;
+    const int G = kp / Pk<T>::L;
+    const int sms = std::max(1, device_sms() / std::max(1, t_pcg_share));
+    const double entries = (double)a.stored * kp;
+    const bool fuse = entries / 2.0 / sms < kFuseClocks<T>;
+    // clocks of a step over all SMs: FP64 FMAs (two per clock), or gathered bytes
+    // (64 per clock)
+    const double work = sizeof(T) == 8 ? (2.0 * entries + 5.0 * a.n * kp) / 2.0
+                                       : 2.0 * entries * sizeof(T) / 64.0;
+    auto units = [&](int nb, int gu) { return (a.nslices + nb - 1) / nb * ((G + gu - 1) / gu); };
+    const int csize = std::min(pcg_small_cluster<T, 1, 1>(),
+                               std::min(pcg_small_cluster<T, 2, 1>(), pcg_small_cluster<T, 2, 2>()));
+    const bool cluster =
+        fuse && csize > 0 && units(csize, 2) <= 2 * NW && work / csize <= kClusterClocks<T>;
+    const int nb = cluster ? csize : std::max(1, std::min(sms, a.nslices));
+    if (!cluster && units(nb, 2) > 2 * NW) return false;
+    // narrow chunks while every warp has one unit at most: more warps at work
+    const int gu = units(nb, 1) <= NW ? 1 : 2, u = units(nb, gu) <= NW ? 1 : 2;
+    auto go = [&](auto GU, auto U) {
+        constexpr int g = decltype(GU)::value, v = decltype(U)::value;
+        if (fuse) launch_pcg_small_form<T, g, v, true>(a, kp, cluster, nb, st);
+        else launch_pcg_small_form<T, g, v, false>(a, kp, cluster, nb, st);
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    if (gu == 1) go(One{}, One{});
+    else if (u == 1) go(Two{}, One{});
+    else go(Two{}, Two{});
+    return true;
+}
+
+constexpr int kMaxBlocksPerSm = 4;
+
+template <typename T, int KP>
+void launch_block_pcg(PcgArgs<T> a, cudaStream_t st) {
+    static PerDevice<int> occupancy;
+    const int bpsm = occupancy.get([] {
+        int b = 0;
+        GCGE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_block_pcg<T, KP>,
+                                                                pcg_threads<T, KP>(), 0));
+        return std::min(b, kMaxBlocksPerSm);
+    });
+    GCGE_REQUIRE(bpsm >= 1, GCGE_ERR_CUDA, "block PCG: kernel does not fit on an SM");
+    const int nb =
+        std::max(1, std::min(bpsm * device_sms() / std::max(1, t_pcg_share), a.nslices));
+    void *args[] = {&a};
+    GCGE_CUDA(cudaLaunchCooperativeKernel((const void *)k_block_pcg<T, KP>, dim3(nb),
+                                          dim3(pcg_threads<T, KP>()), args, 0, st));
+    count_launch();
+}
+
+}  // namespace
+
+template <typename T>
+void block_pcg_rows(PcgWork &wk, const SellPattern &pat, const T *sval, const T *Bv, T *X, T *R,
+                    T *P, T *W, int kp, int k, int max_iter, double rate, double tol, bool rel_tol,
+                    bool x_zero, cudaStream_t st) {
+    constexpr int L = 16 / (int)sizeof(T);
+    GCGE_REQUIRE(k >= 1 && k <= kp && kp <= 40 && kp % L == 0 && k <= kPcgMaxCols, GCGE_ERR_ARG,
+                 "block_pcg: block width");
+    if (pat.n == 0) return;
+    PcgArgs<T> a;
+    a.sp = pat.slice_ptr.p;
+    a.col = pat.col.p;
+    a.val = sval;
+    a.n = pat.n;
+    a.nslices = pat.nslices;
+    a.stored = pat.padded;
+    a.B = Bv;
+    a.X = X;
+    a.R = R;
+    a.P = P;
+    a.W = W;
+    a.k = k;
+    a.max_iter = std::max(0, max_iter);
+    a.rel_tol = rel_tol ? 1 : 0;
+    a.x_zero = x_zero ? 1 : 0;
+    a.rate = rate;
+    a.tol = tol;
+    a.matrix_bytes = (double)pat.nnz * (sizeof(T) + 4) + 4.0 * (pat.n + 1);
+    a.sc = wk.sc.p;
+    a.sync = wk.sync.p;
+    a.stats = wk.stats.p;
+    a.part = wk.part.p;
+    a.timeout_ns = kBarrierTimeoutNs;
+    a.max_polls = kBarrierMaxPolls;
+    a.withhold_last = 0;
+    if (t_pcg_barrier_test.active) {
+        a.timeout_ns = t_pcg_barrier_test.timeout_ns;
+        a.withhold_last = t_pcg_barrier_test.withhold_last;
+    }
+    GCGE_CUDA(cudaMemsetAsync(wk.sync.p, 0, sizeof(PcgSync), st));
+    const bool timed = wk.ev_used + 2 <= 65536;
+    if (timed) {
+        while (wk.ev.size() < wk.ev_used + 2) {
+            cudaEvent_t e;
+            GCGE_CUDA(cudaEventCreate(&e));
+            wk.ev.push_back(e);
+        }
+        GCGE_CUDA(cudaEventRecord(wk.ev[wk.ev_used], st));
+    }
+    if (launch_pcg_small<T>(a, kp, st)) {
+        // (small operators)
+    } else if constexpr (sizeof(T) == 4) {
+        switch (kp) {
+#define GCGE_PCG_CASE(W_)                                     \
+    case W_:                                                  \
+        launch_block_pcg<T, W_>(a, st);                       \
+        break;
+            GCGE_PCG_CASE(4) GCGE_PCG_CASE(8) GCGE_PCG_CASE(12) GCGE_PCG_CASE(16)
+            GCGE_PCG_CASE(20) GCGE_PCG_CASE(24) GCGE_PCG_CASE(28) GCGE_PCG_CASE(32)
+            GCGE_PCG_CASE(36) GCGE_PCG_CASE(40)
+            default: throw CudaError{GCGE_ERR_ARG, "block_pcg: unsupported width"};
+        }
+    } else {
+        switch (kp) {
+            GCGE_PCG_CASE(2) GCGE_PCG_CASE(4) GCGE_PCG_CASE(6) GCGE_PCG_CASE(8)
+            GCGE_PCG_CASE(12) GCGE_PCG_CASE(16) GCGE_PCG_CASE(20) GCGE_PCG_CASE(24)
+            GCGE_PCG_CASE(28) GCGE_PCG_CASE(32) GCGE_PCG_CASE(36) GCGE_PCG_CASE(40)
+#undef GCGE_PCG_CASE
+            default: throw CudaError{GCGE_ERR_ARG, "block_pcg: unsupported width"};
+        }
+    }
+    if (timed) {
+        GCGE_CUDA(cudaEventRecord(wk.ev[wk.ev_used + 1], st));
+        wk.ev_used += 2;
+    }
+    wk.launches++;
+}
+
+}  // namespace gcge
