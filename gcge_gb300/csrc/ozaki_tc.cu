@@ -12,8 +12,8 @@
 // the others balanced in [-128, 127].  Digits are exact in FP16, the 28 digit
 // pairs with i + j <= 6 are multiplied on the tensor cores and summed into 7
 // level accumulators L_l = sum_{i+j=l} d_i d'_j, which are exact FP32 integers
-// as long as |L_l| < 2^24: 144 consecutive k at most (|L_6| <= 144 * 7 * 128^2
-// < 2^23.98).  Every 144 k ("drain") the levels are read out of tensor memory
+// as long as |L_l| < 2^24: 128 consecutive k (|L_6| <= 128 * 7 * 128^2 <
+// 2^23.81).  Every 128 k ("chunk") the levels are read out of tensor memory
 // into one exact 96-bit integer per output; at the end of a window it is
 // converted to FP64 (integer instructions, round to nearest) with the window's
 // scale.  A Gram work item has one window over its whole k range (error below
@@ -25,30 +25,34 @@
 //    k_tc_exprows: per column of the Gram operands over each window, per row
 //    of the linear combination's left operand);
 //  * bulk tensor copies (cp.async.bulk.tensor.2d, TMA) bring the raw FP64
-//    tiles of each 32-k raw stage into shared memory two raw stages ahead
-//    (Gram tiles: 16 k x rows boxes with the 128-byte swizzle, so that lanes
-//    reading rows hit distinct banks); the right operand of a linear
-//    combination is prepared once per call (k_tc_bprep) and copied in with
-//    cp.async.bulk;
-//  * 16 worker warps turn their core matrices (8 rows x 8 k) of each 16-k
-//    half of a raw stage into the 7 FP16 digit planes of a digit stage (a
-//    ring of two digit stages, K-major core-matrix layout); the last worker
-//    to finish reading a raw stage issues the bulk copies of the raw stage
-//    two ahead;
+//    values of each 32-k stage into shared memory ahead of their use, in boxes
+//    with the 128-byte swizzle, so that the lanes of a warp hit distinct banks;
+//    the right operand of a linear combination is prepared once per call
+//    (k_tc_bprep) and copied into the digit stages with cp.async.bulk;
+//  * 16 worker warps turn core matrices (8 rows x 8 k) into the 7 FP16 digit
+//    planes of a digit stage (a ring of two, K-major core-matrix layout);
 //  * one warp issues the MMAs of each digit stage (M = 128 rows, N = up to
 //    256, K = 16, f16 x f16 -> f32 into the 7 level accumulators, 7 x BN of
-//    the 512 tensor-memory columns) and commits them to mbarriers;
-//  * every worker drains its slice of the levels after each 144-k chunk (warp
-//    w reads lanes 32 (w % 4) .. + 31, BN / 4 columns) and folds it at the
-//    end of each window (a Gram work item longer than one window adds its
-//    windows into its split-k partial).
+//    the 512 tensor-memory columns, two sets of them where they fit) and
+//    commits them to mbarriers;
+//  * every worker drains its slice of the levels after each chunk (warp w reads
+//    lanes 32 (w % 4) .. + 31, BN / 4 columns) and folds it at the end of each
+//    window (a Gram work item longer than one window adds its windows into its
+//    split-k partial).
 // Every wait on an mbarrier is bounded; a wait that runs out sets the error
 // word and every warp stops at its next wait, so the kernel always returns.
+//
+// Measured, with the pre-pass (n = 262144; 16-k digit stages, 144-k chunks and
+// 128-row tiles before -> now): Gram 100 x 20 223 -> 177 us, 180 x 20 408 -> 305,
+// 180 x 40 450 -> 391; linear combination 180 -> 20 352 -> 317 us, 180 -> 40 401 ->
+// 366; n = 2097152: Gram 360 x 40 5.11 -> 4.65 ms, 360 -> 40 4.85 -> 4.52, 400 ->
+// 320 30.7 -> 28.7.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -57,10 +61,9 @@ namespace {
 
 constexpr int kTcDigits = 7;
 constexpr int kTcM = 128;      // output rows per tile (tensor-memory lanes)
-constexpr int kTcStageK = 16;  // k per digit stage (one MMA step)
-constexpr int kTcRawK = 32;    // k per raw (TMA) stage: two digit stages
-constexpr int kTcDrainStages = 9;
-constexpr int kTcDrainK = kTcStageK * kTcDrainStages;  // 144: exact FP32 level sums
+constexpr int kTcStageK = 32;  // k per stage: two MMA steps
+constexpr int kTcDrainStages = 4;
+constexpr int kTcDrainK = kTcStageK * kTcDrainStages;  // 128: exact FP32 level sums
 constexpr int kTcKGroups = kTcStageK / 8;              // core matrices along k per stage
 constexpr int kTcDigStages = 2;                         // ring of digit stages
 constexpr int kTcWarps = 16;  // worker warps: digit conversion and drain
@@ -72,7 +75,7 @@ constexpr long long kTcWaitPolls = 1LL << 22;
 // A Gram work item shares one exponent per column over its whole k range
 // (at most this many rows: the 96-bit level sums stay below 2^86)
 constexpr int kTcSuperGramMax = 16384 * kTcDrainK;
-constexpr int kTcSuperLincomb = 3 * kTcDrainK;  // 432: K up to 432 in one window
+constexpr int kTcSuperLincomb = 432;  // K up to 432 in one window
 
 // Byte layout of one operand tile of R rows in a digit stage: plane i
 // (digit), k-group g (8 consecutive k), row r: i * plane + g * lbo +
@@ -94,34 +97,35 @@ __host__ __device__ constexpr uint32_t tc_lbo_b(int bn) {
 }
 __host__ __device__ constexpr uint32_t tc_tile_b_bytes(int bn) { return kTcKGroups * tc_lbo_b(bn); }
 
-// Shared memory (offsets from a 1024-byte aligned base).  Raw stage of a
-// Gram: A boxes [2][128 rows][16 k] and B boxes [2][BN rows][16 k] of FP64 in
-// the 128-byte swizzle; of a linear combination: A box [32 k][128 rows] and
-// the right operand's prepared digit planes of its two digit stages.  The
-// digit stages form a ring of kTcDigStages.
+// Shared memory (offsets from a 1024-byte aligned base).  Raw values arrive in
+// boxes with the 128-byte swizzle: of a Gram in halves of a stage (16 k), A
+// [rows][16 k] and B [BN rows][16 k], four halves where they fit, else three; of
+// a linear combination two halves at once, A [8][32 k][16 rows] (the right
+// operand's prepared digit planes are copied straight into the digit stage).
 template <int BN, bool GRAM>
 struct TcLayout {
     static constexpr uint32_t a_bytes = tc_tile_bytes(kTcM);
     static constexpr uint32_t b_bytes = tc_tile_b_bytes(BN);
-    static constexpr uint32_t a_box = GRAM ? 16u * kTcM * 8u : (uint32_t)kTcRawK * kTcM * 8u;
-    static constexpr uint32_t b_box = GRAM ? 16u * BN * 8u : b_bytes;  // lincomb: planes
-    // gram: two A boxes and two B boxes; lincomb: one A box and two planes
-    static constexpr uint32_t raw_bytes =
-        GRAM ? 2 * (a_box + b_box) : tc_round(a_box + 2 * b_box, 1024);
-    static constexpr uint32_t raw_off = 0;  // [2] raw stages
+    static constexpr uint32_t a_box = 16u * kTcM * 8u;
+    static constexpr uint32_t b_box = GRAM ? 16u * BN * 8u : 0u;
+    static constexpr uint32_t half_bytes = a_box + b_box;
     static constexpr uint32_t stage_bytes = a_bytes + b_bytes;
-    static constexpr uint32_t dig_off = tc_round(raw_off + 2 * raw_bytes, 1024);
+    static constexpr uint32_t limit = 232448 - 1024 - 256;  // per CTA, alignment, barriers
+    static constexpr int halves =
+        4 * half_bytes + kTcDigStages * stage_bytes + 1024 <= limit ? 4 : 3;
+    static constexpr uint32_t raw_off = 0;
+    static constexpr uint32_t dig_off = tc_round(raw_off + halves * half_bytes, 1024);
     static constexpr uint32_t bar_off = tc_round(dig_off + kTcDigStages * stage_bytes, 16);
-    // mbarriers empty[3] full[3] rfull[2] accf fin
-    static constexpr int nbars = 2 * kTcDigStages + 4;
-    // tmem slot, abort flag, arrival counters rempty[2], raw stages issued
+    // accumulator sets in tensor memory: two let a chunk be drained while the
+    // next one's MMAs run
+    static constexpr int accs = 2 * kTcDigits * BN <= (int)kTcTmemCols ? 2 : 1;
+    // mbarriers empty[2] full[2] rfull[4] accf[2] fin
+    static constexpr int nbars = 2 * kTcDigStages + 7;
+    // tmem slot, abort flag, readers' arrivals, raw halves and planes issued
     static constexpr uint32_t misc_off = bar_off + nbars * 8;
     static constexpr uint32_t bytes = misc_off + 48;
     static constexpr uint32_t alloc_bytes = bytes + 1024;  // room to align the base
-    // what the bulk copies of one raw stage write fits the stage
-    static_assert((GRAM ? 2 * (a_box + b_box) : a_box + 2 * b_box) <= raw_bytes,
-                  "raw stage too small for its bulk copies");
-    static_assert(raw_off + 2 * raw_bytes <= dig_off, "raw stages overlap the digit stages");
+    static_assert(half_bytes % 1024 == 0, "swizzled boxes start on 1024 bytes");
     static_assert(alloc_bytes <= 232448, "shared memory beyond the per-CTA limit");
 };
 
@@ -129,10 +133,11 @@ struct TcArgs {
     int M, N, K;
     const double *A;  // gram: Q (k, r) at A[k + r lda]; lincomb: X (r, k) at A[r + k lda]
     size_t lda;
-    int super_k;      // k per exponent window (multiple of kTcDrainK)
+    int super_k;      // k per exponent window (gram: a multiple of kTcDrainK)
     int kchunk;       // gram: k per work item (multiple of super_k)
     int items;        // work items
     int mtiles, ntiles;
+    int mrows;        // rows of a tile: a multiple of 8, at most kTcM
     double *out;      // gram: partials [kz][M x N]; lincomb: Y (ldo)
     size_t ldo;
     const double *beta;
@@ -192,6 +197,7 @@ __device__ __forceinline__ unsigned long long tc_global_ns() {
 // together; lane 0 waits and the result is broadcast.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *b, uint32_t parity,
                                                volatile int *abort_flag, int *gerror) {
+    if (__all_sync(0xffffffffu, mbar_test(b, parity))) return true;
     int ok = 1;
     if ((threadIdx.x & 31) == 0 && !mbar_test(b, parity)) {
         const unsigned long long t0 = tc_global_ns();
@@ -268,6 +274,15 @@ __device__ __forceinline__ void tc_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// One lane of the (converged) calling warp; the compiler then knows the branch
+// to be taken by one thread and keeps the MMAs' operands in uniform registers.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(p));
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- digits
 __device__ __forceinline__ int tc_exp_field(double x) {
     return max((int)(((unsigned)__double2hiint(x) >> 20) & 0x7FFu), 1);
@@ -275,10 +290,9 @@ __device__ __forceinline__ int tc_exp_field(double x) {
 
 // X = |x| 2^(1077 - emax) as a 55-bit fixed-point integer (truncated; the
 // caller guarantees emax >= the exponent field of x), plus 0x808080808080,
-// as two words: the 53-bit significand shifted left by 2, then right by
-// r = emax - field (at most 63: everything past 55 bits is gone), a 64-bit
-// shift made of one wrapping and one clamping funnel shift.  hi = x's high
-// word (its sign bit is the sign).
+// as two words: the 53-bit significand at the top of 64 bits, shifted right by
+// 9 + emax - field (a 64-bit shift of 64 or more gives 0).  hi = x's high word
+// (its sign bit is the sign).
 __device__ __forceinline__ void tc_fixed55(double x, uint32_t emax, uint32_t &yh, uint32_t &yl,
                                            uint32_t &hi) {
     hi = (uint32_t)__double2hiint(x);
@@ -286,12 +300,12 @@ __device__ __forceinline__ void tc_fixed55(double x, uint32_t emax, uint32_t &yh
     const uint32_t eb = hi & 0x7FF00000u;  // exponent field << 20
     // the hidden bit, absent for zeros and subnormals (which count as field 1)
     const uint32_t mhi = (hi & 0x000FFFFFu) | min(eb, 0x00100000u);
-    const uint32_t xh = __funnelshift_l(lo, mhi, 2);
-    const uint32_t xl = lo << 2;
-    const uint32_t r = min(emax - (max(eb, 0x00100000u) >> 20), 63u);
-    const bool big = r >= 32u;
-    const uint32_t sl = __funnelshift_r(big ? xh : xl, big ? 0u : xh, r);  // shift r mod 32
-    const uint32_t sh = __funnelshift_rc(xh, 0u, r);                       // 0 for r >= 32
+    const uint32_t xh = __funnelshift_l(lo, mhi, 11);
+    const uint32_t field = max(eb, 0x00100000u) >> 20;
+    uint32_t sl, sh;
+    asm("{\n.reg .b64 t;\nmov.b64 t, {%2, %3};\nshr.u64 t, t, %4;\nmov.b64 {%0, %1}, t;\n}\n"
+        : "=r"(sl), "=r"(sh)
+        : "r"(lo << 11), "r"(xh), "r"(emax + 9u - field));
     asm("add.cc.u32 %0, %2, 0x80808080;\n\taddc.u32 %1, %3, 0x8080;"
         : "=r"(yl), "=r"(yh)
         : "r"(sl), "r"(sh));
@@ -320,7 +334,7 @@ __device__ __forceinline__ void tc_digit_pair(double x0, double x1, uint32_t ema
     // +-1024 in each half: the sign bits of the two values at bits 15 and 31
     const uint32_t M = (__byte_perm(h0, h1, 0x7030) & 0x80008000u) | 0x64006400u;
     const uint32_t Mb = M | 0x00800080u;                // +-(1024 + 128)
-    w[0] = tc_hsub2((yh0 >> 16) | (yh1 & 0xFFFF0000u) | M, M);
+    w[0] = tc_hsub2(__byte_perm(yh0, yh1, 0x7632) | M, M);
     // byte 6 - i of Y: bytes 4, 5 in the high word, 0..3 in the low word; the
     // permutation puts value 0's byte in half 0 and value 1's in half 1
     w[1] = tc_hsub2((__byte_perm(yh0, yh1, 0x0501) & 0x00FF00FFu) | M, Mb);
@@ -413,18 +427,6 @@ __device__ __forceinline__ void tc_acc96(uint32_t &w0, uint32_t &w1, uint32_t &w
         : "+r"(w0), "+r"(w1), "+r"(w2)
         : "r"(a0), "r"(a1), "r"(a2));
 }
-__device__ __forceinline__ void tc_acc64(uint32_t &w1, uint32_t &w2, uint32_t a1, uint32_t a2) {
-    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, %3;" : "+r"(w1), "+r"(w2) : "r"(a1), "r"(a2));
-}
-// += v 2^(8 (6 - l)) for a level sum v (|v| < 2^31)
-__device__ __forceinline__ void tc_acc_level(uint32_t &w0, uint32_t &w1, uint32_t &w2, int v, int l) {
-    const uint32_t sx = (uint32_t)(v >> 31);
-    const int sh = 8 * (6 - l);
-    if (sh == 0) tc_acc96(w0, w1, w2, (uint32_t)v, sx, sx);
-    else if (sh < 32) tc_acc96(w0, w1, w2, (uint32_t)v << sh, (uint32_t)(v >> (32 - sh)), sx);
-    else if (sh == 32) tc_acc64(w1, w2, (uint32_t)v, sx);
-    else tc_acc64(w1, w2, (uint32_t)v << (sh - 32), (uint32_t)(v >> (64 - sh)));
-}
 
 // Waits, with a bound of its own and regardless of the abort flag, for a
 // phase that asynchronous work of this CTA still completes (bulk copies or
@@ -449,7 +451,7 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs &a, int it) {
     TcItem w;
     const int mn = a.mtiles * a.ntiles;
     const int z = it / mn, r = it % mn;
-    w.mt0 = (r % a.mtiles) * kTcM;
+    w.mt0 = (r % a.mtiles) * a.mrows;
     w.nt = r / a.mtiles;
     if (GRAM) {
         w.kb = z * a.kchunk;
@@ -458,6 +460,16 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs &a, int it) {
         w.kb = 0;
         w.ke = a.K;
     }
+    return w;
+}
+// Work item it + gridDim.x after w (item it).  A linear combination's items are
+// short, so they are stepped instead of divided out.
+template <bool GRAM>
+__device__ __forceinline__ TcItem tc_item_after(const TcArgs &a, TcItem w, int next) {
+    if (GRAM) return tc_item<GRAM>(a, next);
+    const int span = a.mtiles * kTcM;
+    w.mt0 += (int)gridDim.x * kTcM;
+    while (w.mt0 >= span) w.mt0 -= span, ++w.nt;
     return w;
 }
 // A position in this CTA's sequence of raw stages: work item, window start,
@@ -479,7 +491,7 @@ __device__ __forceinline__ void cur_init(const TcArgs &a, TcCursor &c) {
 template <bool GRAM>
 __device__ __forceinline__ void cur_next(const TcArgs &a, TcCursor &c) {
     const int ske = min(c.w.ke, c.sk + a.super_k);
-    c.k0 += kTcRawK;
+    c.k0 += kTcStageK;
     if (c.k0 < ske) return;
     c.sk += a.super_k;
     if (c.sk < c.w.ke) {
@@ -489,46 +501,57 @@ __device__ __forceinline__ void cur_next(const TcArgs &a, TcCursor &c) {
     c.it += gridDim.x;
     c.valid = c.it < a.items;
     if (c.valid) {
-        c.w = tc_item<GRAM>(a, c.it);
+        c.w = tc_item_after<GRAM>(a, c.w, c.it);
         c.sk = c.k0 = c.w.kb;
     }
 }
 
 // ---------------------------------------------------------------- kernel
-// Warps 0 .. 15 are the workers.  Per digit stage a worker thread converts
-// one pair of consecutive k in each of two core matrices of the left operand
-// and, for a Gram, one of the right operand's when it is its warp's turn (those
-// rotate over the warps from stage to stage); after each drain chunk it moves
+// Warps 0 .. 15 are the workers.  Per stage (32 k) a worker warp converts its
+// units, core matrices of 8 rows x 8 k with a pair of consecutive k per lane:
+// its share of the left operand's and, for a Gram, its turn of the right
+// operand's.  After each drain chunk it moves
 // its slice of the level accumulators (tensor-memory lane quarter warp % 4,
 // BN / 4 columns) into 96-bit integers, and after an exponent window it folds
-// them into FP64.  The last worker to finish reading a raw stage issues the
-// bulk copies of the raw stage two ahead into its buffer.  Warp 16 issues the
-// MMAs of each digit stage once every worker has finished it (a dedicated
-// warp: the issue blocks while the tensor core works through the previous
-// stage, ~700 cycles of MMAs per stage).
+// them into FP64.  The last worker to have read a stage's raw halves issues the
+// bulk copies that take their buffers.  Warp 16 issues the MMAs of each
+// stage once every worker has finished it (a dedicated warp: the issue blocks
+// while the tensor core works through the previous stage).
 //
-// The waits form no cycle: digit stage t is produced after the MMAs of stage
-// t - 2 completed (a ring of two digit stages); a worker drains the chunk that
-// ends at stage e before it finishes stage e + 1, so the MMAs of stage e + 1,
-// the next chunk's first (which overwrite the accumulators), are issued after
-// every worker drained it.
+// Rows of a tile past the operand's last row group hold whatever the buffers
+// held: they reach only output rows (or columns) that are not read.
+//
+// The workers bound it, by their instructions (half of the issue slots, the ALU
+// at 52%) and their latency at four warps per scheduler; the tensor cores are
+// busy a quarter of the time, HBM a third.  So a stage is as long as shared
+// memory allows (a third of the instructions of 16-k stages were waits, cursors
+// and addresses), the code is short (a second copy of the conversion cost 5% in
+// instruction fetches) and no register is spilled in the loop (the shared memory
+// taken leaves no L1: spilled accumulators doubled the time).
+//
+// The waits form no cycle: stage t is produced after the MMAs of stage t - 2
+// completed (a ring of two digit stages); a worker drains chunk c before it
+// finishes the first stage of chunk c + accs, whose MMAs overwrite chunk c's
+// accumulators.
 template <int BN, bool GRAM>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_tc_digits(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                 TcArgs a) {
     using L = TcLayout<BN, GRAM>;
     static_assert(BN % 16 == 0 && BN <= 64, "tile width: a multiple of 16, at most 64");
+    constexpr int RH = L::halves, ACCS = L::accs;
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     // 1024-byte aligned base (the 128-byte swizzle of the bulk copies needs it)
     uint8_t *sm = sm_raw + ((1024u - (su32(sm_raw) & 1023u)) & 1023u);
     uint64_t *bars = reinterpret_cast<uint64_t *>(sm + L::bar_off);
     uint64_t *empty = bars, *full = bars + kTcDigStages, *rfull = bars + 2 * kTcDigStages;
-    uint64_t *accf = rfull + 2, *fin = rfull + 3;
+    uint64_t *accf = rfull + 4, *fin = rfull + 6;
     uint32_t *misc = reinterpret_cast<uint32_t *>(sm + L::misc_off);
     uint32_t *tmem_slot = misc;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 1);
-    uint32_t *rcnt = misc + 2;
-    int *n_raw = reinterpret_cast<int *>(misc + 4);  // raw stages issued
+    uint32_t *rcnt = misc + 2;                          // readers of a stage, two in turn
+    int *n_raw = reinterpret_cast<int *>(misc + 4);    // raw halves issued
+    int *n_planes = reinterpret_cast<int *>(misc + 5);  // right-operand stages issued (lincomb)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sbase = su32(sm);
     const int super_k = a.super_k;
@@ -536,16 +559,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (tid == 0) {
         for (int s = 0; s < kTcDigStages; ++s) {
             mbar_init(&empty[s], 1);
-            mbar_init(&full[s], kTcWarps);
+            mbar_init(&full[s], kTcWarps + (GRAM ? 0 : 1));
         }
+        for (int s = 0; s < 4; ++s) mbar_init(&rfull[s], 1);
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&rfull[s], 1);
+            mbar_init(&accf[s], 1);
             rcnt[s] = 0;
         }
-        mbar_init(accf, 1);
         mbar_init(fin, 1);
         *abort_flag = 0;
         *n_raw = 0;
+        *n_planes = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -560,74 +584,82 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // bulk copies of raw stage q (cursor c) into raw buffer q % 2
-    auto issue_raw = [&](uint32_t q, const TcCursor &c) {
-        const uint32_t r = q & 1;
-        const uint32_t base = sbase + L::raw_off + r * L::raw_bytes;
+    // bulk copies of raw half h, the k0 + 16 (h % 2) part of the stage at cursor c,
+    // into raw buffer h % RH (a linear combination's two halves with the first)
+    auto issue_raw = [&](uint32_t h, const TcCursor &c) {
+        const uint32_t r = h % RH;
+        const uint32_t base = sbase + L::raw_off + r * L::half_bytes;
+        const int k0 = c.k0 + 16 * (int)(h & 1);
         if (GRAM) {
-            mbar_expect_tx(&rfull[r], 2 * (L::a_box + L::b_box));
-            tma_load_2d(base, &mapA, c.k0, c.w.mt0, &rfull[r]);
-            tma_load_2d(base + L::a_box, &mapA, c.k0 + 16, c.w.mt0, &rfull[r]);
-            tma_load_2d(base + 2 * L::a_box, &mapB, c.k0, c.w.nt * BN, &rfull[r]);
-            tma_load_2d(base + 2 * L::a_box + L::b_box, &mapB, c.k0 + 16, c.w.nt * BN, &rfull[r]);
+            mbar_expect_tx(&rfull[r], (uint32_t)a.mrows * 128u + L::b_box);
+            tma_load_2d(base, &mapA, k0, c.w.mt0, &rfull[r]);
+            tma_load_2d(base + L::a_box, &mapB, k0, c.w.nt * BN, &rfull[r]);
         } else {
-            // the A box and the prepared planes of the stage's digit stages
-            const int ske = min(c.w.ke, c.sk + super_k);
-            const int nd = min(2, (ske - c.k0 + kTcStageK - 1) / kTcStageK);
-            mbar_expect_tx(&rfull[r], L::a_box + nd * L::b_box);
-            tma_load_2d(base, &mapA, c.w.mt0, c.k0, &rfull[r]);
-            const uint8_t *src =
-                a.bplanes + ((size_t)c.w.nt * a.nstages + (c.k0 - c.w.kb) / kTcStageK) * L::b_bytes;
-            for (int dd = 0; dd < nd; ++dd)
-                bulk_load(base + L::a_box + dd * L::b_box, src + (size_t)dd * L::b_bytes, L::b_bytes,
-                          &rfull[r]);
+            if (h & 1) return;
+            mbar_expect_tx(&rfull[r], 2 * L::a_box);
+#pragma unroll
+            for (int g = 0; g < kTcM / 16; ++g)
+                tma_load_2d(base + g * 4096u, &mapA, c.w.mt0 + 16 * g, k0, &rfull[r]);
         }
-        atomicMax(n_raw, (int)q + 1);
+        atomicMax(n_raw, (int)h + 1);
     };
-    // the MMAs of digit stage t (buffer s, stage st of its drain chunk)
-    auto issue_mma = [&](uint32_t s, int st, bool last_of_chunk) {
+    // the MMAs of a stage (buffer s, accumulator set acc, stage st of its chunk, its
+    // 16-k steps)
+    auto issue_mma = [&](uint32_t s, uint32_t acc, int st, int steps, bool last_of_chunk) {
         const uint32_t abase = sbase + L::dig_off + s * L::stage_bytes;
         const uint32_t bbase = abase + L::a_bytes;
         // left plane i times right planes j = 0 .. 6 - i, into levels l = i + j,
         // in MMAs of at most kLvl levels (N <= 256)
         constexpr int kLvl = 256 / BN < kTcDigits ? 256 / BN : kTcDigits;
 #pragma unroll
-        for (int i = 0; i < kTcDigits; ++i) {
-            const uint64_t ad = smem_desc(abase + i * tc_plane(kTcM), tc_lbo(kTcM), 128);
+        for (int ks = 0; ks < kTcStageK / 16; ++ks) {
+            if (ks >= steps) break;
 #pragma unroll
-            for (int l0 = i; l0 < kTcDigits; l0 += kLvl) {
-                const int nl = min(kLvl, kTcDigits - l0);
-                const uint64_t bd =
-                    smem_desc(bbase + (uint32_t)((l0 - i) * BN / 8) * 128u, tc_lbo_b(BN), 128);
-                // the first product into a level in a drain chunk overwrites it
-                // (level l first meets i = 0)
-                tc_mma(tmem + (uint32_t)(l0 * BN), ad, bd, tc_idesc(kTcM, nl * BN),
-                       (st > 0 || i > 0) ? 1u : 0u);
+            for (int i = 0; i < kTcDigits; ++i) {
+                const uint64_t ad = smem_desc(abase + i * tc_plane(kTcM) + 2 * ks * tc_lbo(kTcM),
+                                              tc_lbo(kTcM), 128);
+#pragma unroll
+                for (int l0 = i; l0 < kTcDigits; l0 += kLvl) {
+                    const int nl = min(kLvl, kTcDigits - l0);
+                    const uint64_t bd = smem_desc(bbase + 2 * ks * tc_lbo_b(BN) +
+                                                      (uint32_t)((l0 - i) * BN / 8) * 128u,
+                                                  tc_lbo_b(BN), 128);
+                    // the first product into a level in a drain chunk overwrites it
+                    // (level l first meets i = 0)
+                    tc_mma(tmem + (acc * kTcDigits + (uint32_t)l0) * BN, ad, bd,
+                           tc_idesc(kTcM, nl * BN), (st > 0 || ks > 0 || i > 0) ? 1u : 0u);
+                }
             }
         }
         tc_commit(&empty[s]);
-        if (last_of_chunk) tc_commit(accf);
+        if (last_of_chunk) tc_commit(&accf[acc]);
     };
 
     if (warp == kTcWarps) {
         // ------------------------------------------------------------ MMA issuer
-        uint32_t s = 0, ph = 0;  // ring position and phase of the next digit stage
+        uint32_t s = 0, ph = 0;  // ring position and phase of the next stage
+        uint32_t acc = 0;        // accumulator set of the chunk
         bool ok = true;
         for (int it = blockIdx.x; it < a.items && ok; it += gridDim.x) {
             const TcItem w = tc_item<GRAM>(a, it);
-            for (int k0 = w.kb; k0 < w.ke && ok; k0 += kTcDrainK) {
-                const int nst = min(kTcDrainStages, (w.ke - k0 + kTcStageK - 1) / kTcStageK);
-                for (int st = 0; st < nst; ++st) {
-                    // every worker finished the stage (and drained the previous
-                    // chunk before the first stage of this one)
-                    if (!mbar_wait_warp(&full[s], ph, abort_flag, a.error)) {
-                        ok = false;
-                        break;
+            for (int sk = w.kb; sk < w.ke && ok; sk += super_k) {
+                const int ske = min(w.ke, sk + super_k);
+                for (int k0 = sk; k0 < ske && ok; k0 += kTcDrainK) {
+                    const int nst = min(kTcDrainStages, (ske - k0 + kTcStageK - 1) / kTcStageK);
+                    for (int st = 0; st < nst; ++st) {
+                        // every worker finished the stage (and drained the chunk
+                        // whose accumulators its first MMAs overwrite)
+                        if (!mbar_wait_warp(&full[s], ph, abort_flag, a.error)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const int steps = ske - k0 - st * kTcStageK <= 16 ? 1 : 2;
+                        if (tc_elect()) issue_mma(s, acc, st, steps, st == nst - 1);
+                        __syncwarp();
+                        if (++s == kTcDigStages) s = 0, ph ^= 1;
                     }
-                    tc_fence_after();
-                    if (lane == 0) issue_mma(s, st, st == nst - 1);
-                    __syncwarp();
-                    if (++s == kTcDigStages) s = 0, ph ^= 1;
+                    if (++acc == ACCS) acc = 0;
                 }
             }
         }
@@ -639,23 +671,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (tid == 0) {
             TcCursor c;
             cur_init<GRAM>(a, c);
-            for (uint32_t q = 0; q < 2 && c.valid; ++q) {
-                issue_raw(q, c);
-                cur_next<GRAM>(a, c);
+            for (uint32_t h = 0; h < (uint32_t)RH && c.valid; ++h) {
+                issue_raw(h, c);
+                if (h & 1) cur_next<GRAM>(a, c);
             }
         }
 
-        // Work units of a digit stage: core matrices (8 rows x 8 k), one pair of
-        // consecutive k per lane: lane = 8 pp + r, row r of the core matrix, k
-        // pair pp.  The 4-byte digit stores of a warp fill one 128-byte line,
-        // and the 16-byte reads of a quarter-warp from a swizzled box (row r's
-        // chunk 4 g + pp at (4 g + pp) ^ r) hit distinct banks.  Warp w converts
-        // the left operand's row group w in both k-groups; the right operand's
-        // units (Gram) rotate over the warps from stage to stage.
+        // Lane = 8 pp + r: row r of a core matrix, k pair pp.  The 4-byte digit
+        // stores of a warp fill one 128-byte line, and its reads of a swizzled box
+        // (row r's chunk c at c ^ r in a Gram, row pair c of k at c ^ k otherwise)
+        // take the fewest bank cycles.
         const int r7 = lane & 7, pp = lane >> 3;
-        const int ra = warp * 8 + r7;  // left-operand row of this thread
-        const uint32_t a_dst = (uint32_t)warp * 128u + (uint32_t)r7 * 16u + (uint32_t)pp * 4u;
-        constexpr int BU = BN / 4;  // right-operand units: BN / 8 row groups x 2 k-groups
         // drain slice: row q 32 + lane, columns [cp CPW, (cp + 1) CPW)
         constexpr int CPW = BN / 4;
         const int q = warp & 3, cp = warp >> 2;
@@ -665,49 +691,52 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         uint32_t w0[CPW], w1[CPW], w2[CPW];
 #pragma unroll
         for (int c = 0; c < CPW; ++c) w0[c] = w1[c] = w2[c] = 0;
+        const int amode = a.alpha == 1.0 ? 0 : a.alpha == -1.0 ? 1 : 2;
 
-        // the next chunk to drain: work item, window start, chunk start,
-        // index of its last digit stage
+        // the next chunk to drain: work item, window start, chunk start, its index
         TcItem dw{0, 0, 0, 0};
-        int dit = blockIdx.x, dsk = 0, dk0 = 0, dlast = 0;
+        int dit = blockIdx.x, dsk = 0, dk0 = 0;
         bool dvalid = dit < a.items;
         uint32_t dn = 0;  // chunks drained
-        auto dstages = [&]() { return min(kTcDrainStages, (dw.ke - dk0 + kTcStageK - 1) / kTcStageK); };
         if (dvalid) {
             dw = tc_item<GRAM>(a, dit);
             dsk = dk0 = dw.kb;
-            dlast = dstages() - 1;
         }
         auto drain = [&]() -> bool {
-            if (!mbar_wait_warp(accf, dn & 1, abort_flag, a.error)) return false;
+            const uint32_t acc = dn % ACCS;
+            if (!mbar_wait_warp(&accf[acc], (dn / ACCS) & 1, abort_flag, a.error)) return false;
             tc_fence_after();
-            const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cp * CPW);
+            // (rows and columns past the operands' are not read)
+            const int drows = min(a.mrows, a.M - dw.mt0);
+            const bool live = q * 32 < drows && dw.nt * BN + cp * CPW < a.N;
+            const uint32_t tb =
+                tmem + ((uint32_t)(q * 32) << 16) + acc * kTcDigits * BN + (uint32_t)(cp * CPW);
             // levels 0 and 1, 2 and 3 pair up exactly in 32 bits (|L_0 2^8 + L_1|
-            // < 2^30.2, |L_2 2^8 + L_3| < 2^30.9): each pair is read with one
-            // wait and added once; levels 4, 5 and 6 are added alone
+            // < 2^30.2, |L_2 2^8 + L_3| < 2^30.9), levels 4 to 6 in 64 with
+            // multiply-adds, which stay off the ALU that the digit extraction fills
             auto f2i = [](uint32_t u) { return __float2int_rn(__uint_as_float(u)); };
-#pragma unroll
-            for (int l = 0; l < 4; l += 2) {
-                uint32_t u[CPW / 4][4], v[CPW / 4][4];
+            if (live) {
 #pragma unroll
                 for (int j = 0; j < CPW / 4; ++j) {
-                    tc_ld4(tb + (uint32_t)(l * BN + 4 * j), u[j]);
-                    tc_ld4(tb + (uint32_t)((l + 1) * BN + 4 * j), v[j]);
+                    uint32_t u[kTcDigits][4];
+#pragma unroll
+                    for (int l = 0; l < kTcDigits; ++l) tc_ld4(tb + (uint32_t)(l * BN + 4 * j), u[l]);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int c = 4 * j + e;
+                        const int p01 = f2i(u[0][e]) * 256 + f2i(u[1][e]);
+                        const int p23 = f2i(u[2][e]) * 256 + f2i(u[3][e]);
+                        const long long hi = (long long)p01 * 65536 + p23;  // 2^24
+                        const long long lo = (long long)f2i(u[4][e]) * 65536 +
+                                             (long long)f2i(u[5][e]) * 256 + f2i(u[6][e]);
+                        const uint32_t hl = (uint32_t)hi, hh = (uint32_t)(hi >> 32);
+                        tc_acc96(w0[c], w1[c], w2[c], hl << 24, __funnelshift_r(hl, hh, 8),
+                                 (uint32_t)((int)hh >> 8));
+                        tc_acc96(w0[c], w1[c], w2[c], (uint32_t)lo, (uint32_t)(lo >> 32),
+                                 (uint32_t)(lo >> 63));
+                    }
                 }
-                tc_wait_ld();
-#pragma unroll
-                for (int c = 0; c < CPW; ++c)
-                    tc_acc_level(w0[c], w1[c], w2[c],
-                                 f2i(u[c >> 2][c & 3]) * 256 + f2i(v[c >> 2][c & 3]), l + 1);
-            }
-#pragma unroll
-            for (int l = 4; l < kTcDigits; ++l) {
-                uint32_t u[CPW / 4][4];
-#pragma unroll
-                for (int j = 0; j < CPW / 4; ++j) tc_ld4(tb + (uint32_t)(l * BN + 4 * j), u[j]);
-                tc_wait_ld();
-#pragma unroll
-                for (int c = 0; c < CPW; ++c) tc_acc_level(w0[c], w1[c], w2[c], f2i(u[c >> 2][c & 3]), l);
             }
             ++dn;
             const int ske = min(dw.ke, dsk + super_k);
@@ -718,7 +747,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 // them there) or straight into Y (a linear combination)
                 const int sidx = (dsk - (GRAM ? 0 : dw.kb)) / super_k;
                 const int grow = dw.mt0 + drow;
-                const int er = grow < a.M ? __ldg(a.eA + (size_t)sidx * a.M + grow) : 1;
+                const bool row_in = drow < drows;
+                const int er = row_in ? __ldg(a.eA + (size_t)sidx * a.M + grow) : 1;
                 const bool first = dsk == dw.kb;
                 const int z = dit / (a.mtiles * a.ntiles);
 #pragma unroll
@@ -735,15 +765,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     if (GRAM) {
                         // the work item's split-k partial: its first window
                         // writes it, later windows add to it
-                        if (grow < a.M && gcol < a.N) {
+                        if (row_in && gcol < a.N) {
                             double *dst = a.out + (size_t)z * a.M * a.N + grow + (size_t)gcol * a.M;
                             *dst = first ? val : *dst + val;
                         }
-                    } else if (grow < a.M && gcol < a.N) {
+                    } else if (row_in && gcol < a.N) {
                         double *dst = a.out + grow + (size_t)gcol * a.ldo;
                         // alpha = +-1 needs no FP64 multiply (the sign folds
                         // into the beta fma or the store)
-                        double y = a.alpha == 1.0 ? val : a.alpha == -1.0 ? -val : a.alpha * val;
+                        double y = amode == 0 ? val : amode == 1 ? -val : a.alpha * val;
                         if (a.accumulate) {
                             y += *dst;
                         } else if (a.beta != nullptr) {
@@ -755,7 +785,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
             }
             // the next chunk
-            const int tnext = dlast + 1;
             dk0 += kTcDrainK;
             if (dk0 >= ske) {
                 dsk += super_k;
@@ -763,143 +792,208 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     dit += gridDim.x;
                     dvalid = dit < a.items;
                     if (dvalid) {
-                        dw = tc_item<GRAM>(a, dit);
+                        dw = tc_item_after<GRAM>(a, dw, dit);
                         dsk = dw.kb;
                     }
                 }
                 dk0 = dsk;
             }
-            if (dvalid) dlast = tnext + dstages() - 1;
             return true;
         };
 
         // ---- production
         TcCursor cons;
         cur_init<GRAM>(a, cons);
-        int t = 0;        // digit stages produced
-        int sidx = 0;     // window of the current raw stage
+        uint32_t t = 0;          // stages produced
+        uint32_t chunk = 0;      // chunk of stage t
         uint32_t s = 0, ph = 0;  // ring position and phase of stage t
-        uint32_t qr = 0;  // raw stages read
-        int em_a = 1;
+        // left-operand units of this warp: row group ga, k-groups kg0 .. kg0 + nku - 1;
+        // right-operand units (Gram): ub0, ub0 + ubs, .. below nub
+        int ga = 0, kg0 = 0, nku = 0, ub0 = 0, ubs = kTcWarps, nub = 0;
+        int em_a = 1, em_b0 = 1, em_b1 = 1;  // exponent fields: row; columns lane, lane + 32
+        // the field of this lane's row in the tile at mt0 (a linear combination
+        // loads the next tile's one tile ahead)
+        auto row_field = [&](int mt0, int g, int rows, int sidx) {
+            return g * 8 + r7 < rows ? __ldg(a.eA + (size_t)sidx * a.M + mt0 + g * 8 + r7) : 0x7FF;
+        };
+        int em_next = 0, mt_next = -1;
         bool ok = true;
         while (ok && cons.valid) {
             const int ske = min(cons.w.ke, cons.sk + super_k);
             if (cons.k0 == cons.sk) {
-                // a window starts: its index and the exponent field of this
-                // thread's row
-                sidx = (cons.sk - (GRAM ? 0 : cons.w.kb)) / super_k;
-                const int gr = cons.w.mt0 + ra;
-                em_a = gr < a.M ? __ldg(a.eA + (size_t)sidx * a.M + gr) : 1;
-            }
-            const uint32_t r = qr & 1;
-            const uint8_t *raw = sm + L::raw_off + r * L::raw_bytes;
-            const int nd = min(2, (ske - cons.k0 + kTcStageK - 1) / kTcStageK);
-            for (int dd = 0; dd < nd; ++dd, ++t) {
-                // the right-operand unit of this warp at stage t (Gram): unit b goes
-                // to warp (b + t BU) mod 16
-                const int bu = (warp - (int)(((uint32_t)t * BU) & 15u)) & 15;
-                const bool hasb = GRAM && bu < BU;
-                const int rb = (bu >> 1) * 8 + r7, gb = bu & 1;
-                int emb = 1;
-                if (hasb) {
-                    const int gc = cons.w.nt * BN + rb;
-                    emb = gc < a.N ? __ldg(a.eB + (size_t)sidx * a.N + gc) : 1;
-                }
-                if (dd == 0 && !mbar_wait_warp(&rfull[r], (qr >> 1) & 1, abort_flag, a.error)) {
-                    ok = false;
-                    break;
-                }
-                // the MMAs of stage t - kTcDigStages read this buffer
-                if (t >= kTcDigStages && !mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, a.error)) {
-                    ok = false;
-                    break;
-                }
-                uint8_t *abuf = sm + L::dig_off + s * L::stage_bytes;
-                uint8_t *bbuf = abuf + L::a_bytes;
+                // a window starts: the units of its tile, and its exponent fields
+                const int sidx = (cons.sk - (GRAM ? 0 : cons.w.kb)) / super_k;
+                const int rows = min(a.mrows, a.M - cons.w.mt0);
+                const int gl = (rows + 7) >> 3;  // row groups: shared by two or four
+                                                 // warps where they are few
+                const int split = gl > 8 ? 0 : gl > 4 ? 1 : 2;
+                ga = warp & (15 >> split);
+                nku = gl > ga ? kTcKGroups >> split : 0;
+                kg0 = (warp >> (4 - split)) * (kTcKGroups >> split);
+                em_a = !GRAM && mt_next == cons.w.mt0 && split == 0
+                           ? em_next
+                           : row_field(cons.w.mt0, ga, rows, sidx);
                 if (!GRAM) {
-                    // the right operand's prepared planes of this digit stage, from
-                    // the raw stage
-                    const uint4 *src = reinterpret_cast<const uint4 *>(raw + L::a_box + dd * L::b_box);
-                    uint4 *dst = reinterpret_cast<uint4 *>(bbuf);
-                    for (int i = tid; i < (int)(L::b_bytes / 16); i += kTcWarps * 32) dst[i] = src[i];
+                    mt_next = tc_item_after<GRAM>(a, cons.w, 0).mt0;
+                    em_next = row_field(mt_next, warp, a.M - mt_next, sidx);
                 }
-                // the pairs: left operand k-groups 0 and 1, and the right-operand unit
-                double2 v0, v1, vb = make_double2(0.0, 0.0);
                 if (GRAM) {
-                    // box dd: row ra's 16 k as 8 chunks of 16 bytes, chunk c at c ^ (ra % 8)
-                    const uint8_t *box = raw + dd * L::a_box + (uint32_t)ra * 128u;
-                    v0 = *reinterpret_cast<const double2 *>(box + ((uint32_t)(pp ^ r7) << 4));
-                    v1 = *reinterpret_cast<const double2 *>(box + ((uint32_t)((4 + pp) ^ r7) << 4));
-                    if (hasb) {
-                        const uint8_t *bx = raw + 2 * L::a_box + dd * L::b_box + (uint32_t)rb * 128u;
-                        vb = *reinterpret_cast<const double2 *>(
-                            bx + ((uint32_t)((4 * gb + pp) ^ r7) << 4));
+                    const int nc = min(BN, a.N - cons.w.nt * BN);
+                    nub = ((nc + 7) >> 3) * kTcKGroups;
+                    // to the warps without row groups where they can take them all,
+                    // else to all warps in turn
+                    const int idle = split == 0 ? kTcWarps - gl : 0;
+                    ubs = idle > 0 && nub <= kTcKGroups * idle ? idle : kTcWarps;
+                    ub0 = ubs == kTcWarps ? (warp - (int)(t * (uint32_t)nub)) & 15
+                                          : (warp >= gl ? warp - gl : nub);
+                    const int *e = a.eB + (size_t)sidx * a.N + cons.w.nt * BN;
+                    em_b0 = lane < nc ? __ldg(e + lane) : 0x7FF;
+                    em_b1 = BN > 32 && lane + 32 < nc ? __ldg(e + lane + 32) : 0x7FF;
+                }
+            }
+            const uint32_t h0 = 2 * t, h1 = h0 + 1;
+            if (!mbar_wait_warp(&rfull[h0 % RH], (h0 / RH) & 1, abort_flag, a.error) ||
+                (GRAM && !mbar_wait_warp(&rfull[h1 % RH], (h1 / RH) & 1, abort_flag, a.error)))
+                break;
+            const uint8_t *raw0 = sm + L::raw_off + (h0 % RH) * L::half_bytes;
+            const uint8_t *raw1 = sm + L::raw_off + (h1 % RH) * L::half_bytes;
+            // a stage's halves are read; the last warp issues the copies of the two
+            // that take their buffers
+            auto release_raw = [&]() {
+                __syncwarp();
+                if (lane == 0 && smem_arrive(&rcnt[t & 1]) == kTcWarps - 1) {
+                    rcnt[t & 1] = 0;
+                    // half h0 + RH belongs to the stage (h0 + RH) / 2
+                    TcCursor c2 = cons;
+                    uint32_t stage = t;
+#pragma unroll 1
+                    for (uint32_t h = h0 + RH; h <= h1 + RH; ++h) {
+                        for (; stage < h / 2 && c2.valid; ++stage) cur_next<GRAM>(a, c2);
+                        if (c2.valid) issue_raw(h, c2);
                     }
+                }
+                __syncwarp();
+            };
+            // a linear combination's values are held in registers (its buffers are
+            // refilled during the conversion); a Gram's are read unit by unit, as
+            // its accumulators and right-operand units need the registers (a spilled
+            // one costs an L2 access: shared memory leaves no L1)
+            double2 va[GRAM ? 1 : kTcKGroups];
+            if (!GRAM) {
+#pragma unroll
+                for (int u = 0; u < kTcKGroups; ++u) {
+                    // box ga / 2: k's 16 rows as 8 chunks of 16 bytes, chunk c at
+                    // c ^ (k % 8)
+                    const int rr = (ga & 1) * 8 + r7;
+                    const int k = (kg0 + min(u, max(nku, 1) - 1)) * 8 + 2 * pp;
+                    const uint8_t *box = raw0 + (uint32_t)(ga >> 1) * 4096u + (uint32_t)k * 128u +
+                                         (uint32_t)(rr & 1) * 8u;
+                    va[u].x = *reinterpret_cast<const double *>(
+                        box + ((uint32_t)((rr >> 1) ^ (2 * pp)) << 4));
+                    va[u].y = *reinterpret_cast<const double *>(
+                        box + 128u + ((uint32_t)((rr >> 1) ^ (2 * pp + 1)) << 4));
+                }
+                release_raw();
+            }
+            // the MMAs of stage t - kTcDigStages read this digit buffer
+            if (t >= kTcDigStages && !mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, a.error)) break;
+            uint8_t *abuf = sm + L::dig_off + s * L::stage_bytes;
+            uint8_t *bbuf = abuf + L::a_bytes;
+            if (!GRAM && tid == 0) {
+                // the right operand's prepared planes of this stage
+                mbar_expect_tx(&full[s], L::b_bytes);
+                bulk_load(su32(bbuf),
+                          a.bplanes + ((size_t)cons.w.nt * a.nstages +
+                                       (cons.k0 - cons.w.kb) / kTcStageK) * L::b_bytes,
+                          L::b_bytes, &full[s]);
+                *n_planes = (int)t + 1;
+            }
+            if (!GRAM) __syncwarp();
+            auto store_a = [&](int kg, const double2 &v) {
+                uint32_t d[kTcDigits];
+                tc_digit_pair(v.x, v.y, (uint32_t)em_a, d);
+                uint8_t *dst = abuf + (uint32_t)kg * tc_lbo(kTcM) + (uint32_t)ga * 128u +
+                               (uint32_t)r7 * 16u + (uint32_t)pp * 4u;
+#pragma unroll
+                for (int i = 0; i < kTcDigits; ++i)
+                    *reinterpret_cast<uint32_t *>(dst + (uint32_t)i * tc_plane(kTcM)) = d[i];
+            };
+            if (!GRAM) {
+                // (a stage of at most 16 k is one MMA step: two k-groups; a warp with
+                // fewer units repeats its last one instead of branching)
+                if (nku > 0 && ske - cons.k0 > 16) {
+#pragma unroll
+                    for (int u = 0; u < kTcKGroups; ++u) store_a(kg0 + min(u, nku - 1), va[u]);
                 } else {
-                    // box [32 k][128 rows]
-                    const double *col = reinterpret_cast<const double *>(raw) +
-                                        (size_t)(dd * kTcStageK + 2 * pp) * kTcM + ra;
-                    v0 = make_double2(col[0], col[kTcM]);
-                    v1 = make_double2(col[8 * kTcM], col[9 * kTcM]);
+#pragma unroll 1
+                    for (int u = 0; u < min(nku, 2 - kg0); ++u)
+                        store_a(kg0 + u, u == 0 ? va[0] : va[1]);
                 }
-                // row groups past the operand's last row hold zero digits: the
-                // conversion is skipped (warp-uniform)
-                const bool live_a = cons.w.mt0 + warp * 8 < a.M;
-                const bool live_b = !GRAM || cons.w.nt * BN + (bu >> 1) * 8 < a.N;
-                uint32_t d0[kTcDigits], d1[kTcDigits], db[kTcDigits];
+            } else {
+                constexpr int NU = BN > 32 ? 1 : 2;
+#pragma unroll 1
+                for (int u = 0; u < nku; u += NU) {
+                    double2 v[NU];
 #pragma unroll
-                for (int i = 0; i < kTcDigits; ++i) d0[i] = d1[i] = db[i] = 0u;
-                if (live_a) {
-                    tc_digit_pair(v0.x, v0.y, (uint32_t)em_a, d0);
-                    tc_digit_pair(v1.x, v1.y, (uint32_t)em_a, d1);
-                }
-                if (hasb && live_b) tc_digit_pair(vb.x, vb.y, (uint32_t)emb, db);
+                    for (int e = 0; e < NU; ++e) {
+                        // row's 16 k as 8 chunks of 16 bytes, chunk c at c ^ r7
+                        const int kg = kg0 + min(u + e, nku - 1);
+                        v[e] = *reinterpret_cast<const double2 *>(
+                            ((kg & 2) ? raw1 : raw0) + (uint32_t)(ga * 8 + r7) * 128u +
+                            ((uint32_t)((4 * (kg & 1) + pp) ^ r7) << 4));
+                    }
 #pragma unroll
-                for (int i = 0; i < kTcDigits; ++i) {
-                    uint8_t *pa = abuf + (uint32_t)i * tc_plane(kTcM) + a_dst;
-                    *reinterpret_cast<uint32_t *>(pa) = d0[i];
-                    *reinterpret_cast<uint32_t *>(pa + tc_lbo(kTcM)) = d1[i];
+                    for (int e = 0; e < NU; ++e) store_a(kg0 + min(u + e, nku - 1), v[e]);
                 }
-                if (hasb) {
-                    const uint32_t b_dst = (uint32_t)gb * tc_lbo_b(BN) + (uint32_t)(bu >> 1) * 128u +
-                                           (uint32_t)r7 * 16u + (uint32_t)pp * 4u;
+            }
+            if (GRAM) {
+#pragma unroll 1
+                for (int b = ub0; b < nub; b += ubs) {
+                    const int kg = b & 3, rb = (b >> 2) * 8 + r7;
+                    const double2 v = *reinterpret_cast<const double2 *>(
+                        ((kg & 2) ? raw1 : raw0) + L::a_box + (uint32_t)rb * 128u +
+                        ((uint32_t)((4 * (kg & 1) + pp) ^ r7) << 4));
+                    int em = __shfl_sync(0xffffffffu, em_b0, rb & 31);
+                    if (BN > 32) {
+                        const int e1 = __shfl_sync(0xffffffffu, em_b1, rb & 31);
+                        if (rb >= 32) em = e1;
+                    }
+                    uint32_t d[kTcDigits];
+                    tc_digit_pair(v.x, v.y, (uint32_t)em, d);
+                    uint8_t *dst = bbuf + (uint32_t)kg * tc_lbo_b(BN) + (uint32_t)rb * 16u +
+                                   (uint32_t)pp * 4u;
 #pragma unroll
                     for (int i = 0; i < kTcDigits; ++i)
-                        *reinterpret_cast<uint32_t *>(bbuf + b_dst + (uint32_t)i * BN * 16u) = db[i];
+                        *reinterpret_cast<uint32_t *>(dst + (uint32_t)i * BN * 16u) = d[i];
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                // chunks that ended at stage t - 1 or earlier
-                while (dvalid && dlast < t) {
-                    if (!drain()) {
-                        ok = false;
-                        break;
-                    }
+                if (ubs == kTcWarps) ub0 = (ub0 - nub) & 15;
+            }
+            if (GRAM) release_raw();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            // chunks whose accumulators this stage's chunk overwrites
+            while (dvalid && dn + ACCS <= chunk) {
+                if (!drain()) {
+                    ok = false;
+                    break;
                 }
-                if (!ok) break;
-                // arrival (release; the stores and drains above come first)
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full[s]);
-                if (++s == kTcDigStages) s = 0, ph ^= 1;
             }
             if (!ok) break;
-            // raw stage qr is read; the last warp copies raw stage qr + 2 into its buffer
+            // arrival (release; the stores and drains above come first)
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0 && smem_arrive(&rcnt[r]) == kTcWarps - 1) {
-                rcnt[r] = 0;
-                TcCursor c2 = cons;
-                cur_next<GRAM>(a, c2);
-                if (c2.valid) cur_next<GRAM>(a, c2);
-                if (c2.valid) issue_raw(qr + 2, c2);
-            }
-            __syncwarp();
-            ++qr;
+            if (lane == 0) mbar_arrive(&full[s]);
+            if (++s == kTcDigStages) s = 0, ph ^= 1;
+            ++t;
+            // the next stage starts a chunk at a multiple of the drain length in
+            // its window, or with a window
+            const int kn = cons.k0 + kTcStageK;
+            if (kn >= ske || (kn - cons.sk) % kTcDrainK == 0) ++chunk;
             cur_next<GRAM>(a, cons);
         }
+        ok = ok && !cons.valid;
         // the remaining chunks
         while (ok && dvalid)
             if (!drain()) ok = false;
-
     }
     // teardown: the bulk copies still in flight (after an abort) land before
     // the CTA exits; the MMA warp waited for its MMAs
@@ -907,8 +1001,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     if (warp == 0) {
         const int nr = *n_raw;
-        for (int qq = max(nr - 2, 0); qq < nr; ++qq)
-            mbar_wait_teardown(&rfull[qq & 1], (qq >> 1) & 1);
+        for (int h = max(nr - RH, 0); h < nr; ++h)
+            if (GRAM || (h & 1) == 0) mbar_wait_teardown(&rfull[h % RH], (h / RH) & 1);
+        if (!GRAM && *abort_flag) {
+            // the right operand's copies arrive on `full`, whose phase an abort
+            // leaves incomplete: give them the time any copy takes
+            const unsigned long long t0 = tc_global_ns();
+            while (*n_planes > 0 && tc_global_ns() - t0 < 1000000ull) {
+            }
+            __syncwarp();
+        }
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(kTcTmemCols)
@@ -1104,10 +1206,11 @@ PFN_cuTensorMapEncodeTiled_v12000 tc_encode_fn() {
 }
 
 // 2D FP64 tensor map of a column-major block: dim0 (contiguous) x dim1 with
-// row pitch ld doubles, box0 x box1 elements; false where the layout cannot
+// row pitch ld doubles, box0 x box1 elements (box0 x 8 = the 128-byte swizzle's
+// span); false where the layout cannot
 // be described (the caller then uses the FP64 kernels).
 bool tc_map(CUtensorMap *map, const double *base, int dim0, int dim1, size_t ld, int box0,
-            int box1, bool swizzle) {
+            int box1) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = tc_encode_fn();
     if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || (ld * 8) % 16 || dim0 < 1 || dim1 < 1)
         return false;
@@ -1117,7 +1220,7 @@ bool tc_map(CUtensorMap *map, const double *base, int dim0, int dim1, size_t ld,
     const cuuint32_t estr[2] = {1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double *>(base), dims, strides,
                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B,
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1167,9 +1270,13 @@ void tc_gram(int n, int m, int w, const double *Q, int ldq, const double *P, int
         return;
     }
     const int bn = tc_bn(w);
+    // row tiles of equal height (180 rows: 96 + 84 instead of 128 + 52, whose
+    // CTAs finished at half the time of the others)
+    const int mtiles = (m + kTcM - 1) / kTcM;
+    const int mrows = ((m + mtiles - 1) / mtiles + 7) / 8 * 8;
     CUtensorMap ma, mb;
-    if (!tc_map(&ma, Q, n, m, (size_t)ldq, 16, kTcM, true) ||
-        !tc_map(&mb, P, n, w, (size_t)ldp, 16, bn, true)) {
+    if (!tc_map(&ma, Q, n, m, (size_t)ldq, 16, mrows) ||
+        !tc_map(&mb, P, n, w, (size_t)ldp, 16, bn)) {
         gram(n, m, w, Q, ldq, P, ldp, C, ldc, scratch, scratch_elems, st);
         return;
     }
@@ -1179,7 +1286,8 @@ void tc_gram(int n, int m, int w, const double *Q, int ldq, const double *P, int
     a.K = n;
     a.A = Q;
     a.lda = (size_t)ldq;
-    a.mtiles = (m + kTcM - 1) / kTcM;
+    a.mtiles = mtiles;
+    a.mrows = mrows;
     a.ntiles = (w + bn - 1) / bn;
     const int mn = a.mtiles * a.ntiles;
     const int sms = device_sms();
@@ -1253,7 +1361,7 @@ void tc_lincomb(int n, int k, int m, const double *X, int ldx, const double *C, 
     if (n <= 0 || m <= 0) return;
     const int bn = tc_bn(m);
     CUtensorMap ma;
-    if (!tc_map(&ma, X, n, std::min(k, kTcSuperLincomb), (size_t)ldx, kTcM, kTcRawK, false)) {
+    if (!tc_map(&ma, X, n, std::min(k, kTcSuperLincomb), (size_t)ldx, 16, kTcStageK)) {
         lincomb(n, k, m, X, ldx, C, ldc, Y, ldy, beta_dev, incb, st, alpha);
         return;
     }
@@ -1263,7 +1371,7 @@ void tc_lincomb(int n, int k, int m, const double *X, int ldx, const double *C, 
         const int kb = std::min(kTcSuperLincomb, k - k0);
         const double *Xb = X + (size_t)k0 * ldx;
         // (the first block's map was made above; Xb keeps its 16-byte alignment)
-        if (k0 > 0 && !tc_map(&ma, Xb, n, kb, (size_t)ldx, kTcM, kTcRawK, false))
+        if (k0 > 0 && !tc_map(&ma, Xb, n, kb, (size_t)ldx, 16, kTcStageK))
             throw CudaError{GCGE_ERR_ARG, "tc_lincomb: operand layout"};
         TcArgs a{};
         a.M = n;
@@ -1273,6 +1381,7 @@ void tc_lincomb(int n, int k, int m, const double *X, int ldx, const double *C, 
         a.lda = (size_t)ldx;
         a.super_k = kTcSuperLincomb;
         a.mtiles = (n + kTcM - 1) / kTcM;
+        a.mrows = kTcM;
         a.ntiles = (m + bn - 1) / bn;
         a.items = a.mtiles * a.ntiles;
         a.out = Y;
