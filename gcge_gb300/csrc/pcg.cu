@@ -34,6 +34,9 @@ __global__ void k_col_to_rows(int n, int k, int kp, const S *__restrict__ X, int
         Y[t] = (i < n && c < k) ? (T)X[i + (size_t)c * ldx] : T(0);
     }
 }
+// add: Y += X where X is finite.  On an indefinite operator a column of the FP32
+// correction can leave the range of its type (a nearly vanishing p^T S p); such
+// a column of Y stays as it was instead of spoiling the block it belongs to.
 template <typename T, typename D>
 __global__ void k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y,
                               int ldy, int add) {
@@ -43,7 +46,7 @@ __global__ void k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *
         const int c = (int)(t / n), i = (int)(t % n);
         const D v = (D)X[blk_index<T>(i, c, kp)];
         D &y = Y[i + (size_t)c * ldy];
-        y = add ? y + v : v;
+        y = add ? (isfinite(v) ? y + v : y) : v;
     }
 }
 
