@@ -825,15 +825,20 @@ int sym_eig(EigWork &wk, int s, const double *M, int ld, double *eval_host, doub
     count_launch(2);
     const int lds = s;
     double *X = wk.X.p, *Xn = wk.X2.p;
-    // s x s products of the refinement: X^T P (ld s) and A B (ld of A given)
+    // s x s products of the refinement: X^T P (ld s) and A B (ld of A given), on
+    // the digit kernels from the size where these are faster than the FP64 units
+    // (GB300, digits against FP64: X^T P 37 against 16 us at s = 180, 42 against
+    // 113 at 400; A B 51 against 16 and 81 against 113)
+    const double flops = 2.0 * s * s * s;
+    const bool digit_gram = emulated && flops > 2.8e7, digit_lincomb = emulated && flops > 6e7;
     auto sgram = [&](const double *P, double *C) {
-        if (emulated)
+        if (digit_gram)
             oz_gram(s, s, s, X, lds, P, lds, C, lds, wk.gscr.p, wk.gscr.n, st);
         else
             gram(s, s, s, X, lds, P, lds, C, lds, wk.gscr.p, wk.gscr.n, st);
     };
     auto slincomb = [&](const double *A, int lda, const double *B, double *Y, int ldy) {
-        if (emulated)
+        if (digit_lincomb)
             oz_lincomb(s, s, s, A, lda, B, lds, Y, ldy, nullptr, 0, st, 1.0, wk.ozb.p, wk.ozb.n);
         else
             lincomb(s, s, s, A, lda, B, lds, Y, ldy, nullptr, 0, st);

@@ -165,19 +165,34 @@ enum { PH_CHECK = 0, PH_P, PH_RR, PH_RRW, PH_EIG, PH_RV, PH_W, PH_LINSOL, PH_X, 
 // below it for nev up to ~300 - therefore stay FP64; they cost next to
 // nothing.
 constexpr int kDigitMinRows = 1024;
+// Below this many flops the FP64 units are faster than the digit kernel with
+// its pre-passes and launches (GB300, digits against FP64: Gram 4160 x 40 x 6 25
+// against 10 us, 16384 x 60 x 8 27 both, 35937 x 60 x 20 39 against 93; linear
+// combination 19 against 6, 21 against 19, 35 against 77).  The Cholesky-QR
+// products of a block with itself take the digit kernel at every size
+// (self): the digit combination with R^-1 is what bounds the accuracy of a mixed
+// solve near its attainable residual, and with it when such a solve
+// goes over to FP64.
+constexpr double kDigitMinFlops = 1.2e7;
+
+static bool use_digits(const SolverCtx &c, int n, int m, int w, bool self) {
+    return c.precision == GCGE_PREC_MIXED && !c.escalated && n >= kDigitMinRows &&
+           (self || 2.0 * n * m * w >= kDigitMinFlops);
+}
 
 static void dgram(const SolverCtx &c, int n, int m, int w, const double *Q, int ldq,
                   const double *P, int ldp, double *C, int ldc, double *scratch, size_t elems,
-                  cudaStream_t st, TcExpCache *qcache = nullptr) {
-    if (c.precision == GCGE_PREC_MIXED && !c.escalated && n >= kDigitMinRows)
+                  cudaStream_t st, TcExpCache *qcache = nullptr, bool self = false) {
+    if (use_digits(c, n, m, w, self))
         oz_gram(n, m, w, Q, ldq, P, ldp, C, ldc, scratch, elems, st, qcache);
     else
         gram(n, m, w, Q, ldq, P, ldp, C, ldc, scratch, elems, st);
 }
 static void dlincomb(const SolverCtx &c, int n, int k, int m, const double *X, int ldx,
                      const double *C, int ldc, double *Y, int ldy, const double *beta, int incb,
-                     cudaStream_t st, double alpha = 1.0, TcExpCache *xcache = nullptr) {
-    if (c.precision == GCGE_PREC_MIXED && !c.escalated && n >= kDigitMinRows)
+                     cudaStream_t st, double alpha = 1.0, TcExpCache *xcache = nullptr,
+                     bool self = false) {
+    if (use_digits(c, n, k, m, self))
         oz_lincomb(n, k, m, X, ldx, C, ldc, Y, ldy, beta, incb, st, alpha, c.ozb.p, c.ozb.n,
                    xcache);
     else
@@ -255,7 +270,8 @@ int borth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int start, 
                 if (!(pass == 0 && bx1_kept)) applyB(X1, ldx, c.T2.p, ld, k);
                 BX1 = c.T2.p;
             }
-            dgram(c, nrows, k, k, X1, ldx, BX1, useB ? ld : ldx, c.dC.p, k, c.gscr.p, c.gscr.n, st);
+            dgram(c, nrows, k, k, X1, ldx, BX1, useB ? ld : ldx, c.dC.p, k, c.gscr.p, c.gscr.n, st,
+                  nullptr, true);
             GCGE_CUDA(cudaMemcpyAsync(c.hbuf.p, c.dC.p, sizeof(double) * k * k,
                                       cudaMemcpyDeviceToHost, st));
             GCGE_CUDA(cudaStreamSynchronize(st));
@@ -308,7 +324,8 @@ int borth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int start, 
             if (kk > 0) {
                 GCGE_CUDA(cudaMemcpyAsync(c.dC.p, Cf, sizeof(double) * k * kk,
                                           cudaMemcpyHostToDevice, st));
-                dlincomb(c, nrows, k, kk, X1, ldx, c.dC.p, k, c.T1.p, ld, nullptr, 0, st);
+                dlincomb(c, nrows, k, kk, X1, ldx, c.dC.p, k, c.T1.p, ld, nullptr, 0, st, 1.0,
+                         nullptr, true);
                 copy_cols(nrows, kk, c.T1.p, ld, X1, ldx, st);
             }
             k = kk;
