@@ -5,11 +5,12 @@
 // GB300 issues FP64 at ~1/58 of its FP32 rate, so an FP64 Jacobi on one SM
 // would take tens of milliseconds for s = 200.  The solver therefore
 //   1. runs a parallel-order (round-robin) two-sided cyclic Jacobi in FP32,
-//      logging each round's rotations: for s >= 88 in a cluster of 8 CTAs
-//      whose shared memories hold the matrix rows of the pairs each CTA owns
-//      (distributed shared memory; rows move between neighbouring CTAs as the
-//      round-robin order advances), else in one 1024-thread CTA with the
-//      packed upper triangle in shared memory;
+//      logging each round's rotations: up to s = 104 in one CTA with the matrix
+//      in its shared memory, above in a cluster of 8 CTAs whose shared memories
+//      hold the matrix rows of the pairs each CTA owns (distributed shared
+//      memory; rows move between neighbouring CTAs as the round-robin order
+//      advances; where no cluster can be placed, in one 1024-thread CTA with
+//      the packed upper triangle);
 //   2. rebuilds the eigenvector matrix from the rotation log with one warp
 //      per row (rows of V = J_1 J_2 ... J_T are independent);
 //   3. refines eigenvectors and eigenvalues to FP64 accuracy with the
@@ -218,6 +219,162 @@ k_jacobi32(int s, const double *__restrict__ M, int ldm, float4 *__restrict__ lo
     }
 }
 
+// ---------------------------------------------------------------- one-CTA Jacobi on the full matrix
+// The same rotations in the same order as k_jacobi32 on the full s x s matrix
+// (no index of a pair needs sorting) in place.  A round: thread k < np computes
+// the rotation of pair k, while every thread loads its (at most IT) 2x2 blocks
+// of the pair grid; after a barrier the threads update their blocks; a second
+// barrier ends the round.  A thread keeps its blocks' pair numbers i, j over all
+// rounds, and round r pairs r - k with r + k (mod m - 1) and m - 1 with r: a
+// warp's blocks run along a row (m is even, so the pairs' diagonal and
+// off-diagonal entries have odd strides as well: no bank conflicts).  This is the
+// circle method on reversed indices, so k_apply_circle reads the log.
+// The round is bound by its chain of latencies, pivot entries -> rotation ->
+// table -> update, about 400 clocks at s = 64, and beyond that by the one SM's
+// shared-memory accesses, eight a block.  GB300, kernel alone, k_jacobi32, the
+// cluster kernel and this one: s = 30 66, 74, 29 us; s = 64 166, 151, 85 us;
+// s = 96 391, 254, 229 us; s = 112 513, 307, 347 us: hence kJacCtaMax.  (Every warp
+// computing all rotations for itself, with two copies of the matrix and one
+// barrier: s = 30 28, s = 64 107 us.)
+constexpr int kJacCtaMax = 104;  // np^2 blocks: at most 3 a thread
+
+size_t jacobi_cta_smem_bytes(int s) {
+    const int m = jac_m(s);
+    return (size_t)m * m * sizeof(float);
+}
+
+template <int IT>
+__global__ void __launch_bounds__(kJacobiThreads, 1)
+k_jacobi_cta(int s, const double *__restrict__ M, int ldm, float2 *__restrict__ log,
+             int max_rounds, int *__restrict__ info) {
+    extern __shared__ float A[];  // m x m; the padding index of an odd s has zero entries
+    __shared__ float red[2][32][2];
+    __shared__ float2 tab[kJacCtaMax / 2];  // c, s of the round's pairs
+    const int m = jac_m(s), np = m / 2, m1 = m - 1;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
+    for (int idx = t; idx < m * m; idx += blockDim.x) {
+        const int x = idx / m, y = idx - x * m;
+        float v = 0.0f;
+        if (x < s && y < s) v = (float)(0.5 * (M[x + (size_t)y * ldm] + M[y + (size_t)x * ldm]));
+        A[idx] = v;
+    }
+    // the thread's blocks (row pair, column pair)
+    int bi[IT], bj[IT];
+#pragma unroll
+    for (int u = 0; u < IT; ++u) {
+        const int b = t + u * blockDim.x;
+        bi[u] = b < np * np ? b / np : 0;
+        bj[u] = b < np * np ? b - bi[u] * np : 0;
+    }
+    // indices of pair k in round r
+    auto top = [&](int k, int r) {
+        const int v = r - k;
+        return k == 0 ? m1 : (v < 0 ? v + m1 : v);
+    };
+    auto bot = [&](int k, int r) {
+        const int v = r + k;
+        return v >= m1 ? v - m1 : v;
+    };
+    __syncthreads();
+    int round = 0, sweep = 0, converged = 0;
+    for (sweep = 0; sweep < kMaxSweeps && round + m1 <= max_rounds; ++sweep) {
+        // stop when the off-diagonal mass is at the FP32 noise level
+        float off = 0.0f, tot = 0.0f;
+        for (int x = warp; x < m; x += nwarps)
+            for (int y = lane; y < m; y += 32) {
+                const float v = A[x * m + y] * A[x * m + y];
+                tot += v;
+                if (x != y) off += v;
+            }
+        for (int o = 16; o > 0; o >>= 1) {
+            off += __shfl_xor_sync(0xffffffffu, off, o);
+            tot += __shfl_xor_sync(0xffffffffu, tot, o);
+        }
+        if (lane == 0) {
+            red[sweep & 1][warp][0] = off;
+            red[sweep & 1][warp][1] = tot;
+        }
+        __syncthreads();
+        off = tot = 0.0f;
+        for (int w = 0; w < nwarps; ++w) {
+            off += red[sweep & 1][w][0];
+            tot += red[sweep & 1][w][1];
+        }
+        if (off <= kOffTol * kOffTol * tot) {  // the same sums in every thread
+            converged = 1;
+            break;
+        }
+        for (int r = 0; r < m1; ++r) {
+            if (t < np) {
+                const int p = top(t, r), q = bot(t, r);
+                const float app = A[p * m + p], aqq = A[q * m + q], apq = A[p * m + q];
+                float c = 1.0f, sv = 0.0f;
+                const float thr = kRotTol * sqrtf(fabsf(app) * fabsf(aqq));
+                if (fabsf(apq) > thr && fabsf(apq) > 1e-30f) {
+                    // (an infinite tau^2 gives the rotation 0, as it should; tau = 0
+                    // turns towards the larger index whichever of p, q that is)
+                    const float tau = (aqq - app) / (2.0f * apq);
+                    const float tt = ((p < q ? tau >= 0.0f : tau > 0.0f) ? 1.0f : -1.0f) /
+                                     (fabsf(tau) + sqrtf(fmaf(tau, tau, 1.0f)));
+                    c = rsqrtf(1.0f + tt * tt);
+                    sv = tt * c;
+                }
+                tab[t] = make_float2(c, sv);
+                log[(size_t)round * np + t] = make_float2(c, sv);
+            }
+            float d[IT][4];
+#pragma unroll
+            for (int u = 0; u < IT; ++u) {
+                const float *rt = A + top(bi[u], r) * m, *rb = A + bot(bi[u], r) * m;
+                const int p = top(bj[u], r), q = bot(bj[u], r);
+                d[u][0] = rt[p];
+                d[u][1] = rt[q];
+                d[u][2] = rb[p];
+                d[u][3] = rb[q];
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < IT; ++u) {
+                if (t + u * (int)blockDim.x >= np * np) break;
+                const float2 ei = tab[bi[u]], ej = tab[bj[u]];
+                const float t11 = ei.x * d[u][0] - ei.y * d[u][2];
+                const float t12 = ei.x * d[u][1] - ei.y * d[u][3];
+                const float t21 = ei.y * d[u][0] + ei.x * d[u][2];
+                const float t22 = ei.y * d[u][1] + ei.x * d[u][3];
+                float *rt = A + top(bi[u], r) * m, *rb = A + bot(bi[u], r) * m;
+                const int p = top(bj[u], r), q = bot(bj[u], r);
+                const bool zero = bi[u] == bj[u] && ei.y != 0.0f;
+                rt[p] = t11 * ej.x - t12 * ej.y;
+                rt[q] = zero ? 0.0f : t11 * ej.y + t12 * ej.x;
+                rb[p] = zero ? 0.0f : t21 * ej.x - t22 * ej.y;
+                rb[q] = t21 * ej.y + t22 * ej.x;
+            }
+            __syncthreads();
+            ++round;
+        }
+    }
+    if (t == 0) {
+        info[0] = round;
+        info[1] = sweep;
+        info[2] = converged;
+    }
+}
+
+template <int IT>
+static void launch_jacobi_cta(int s, const double *M, int ldm, float2 *log, int max_rounds,
+                              int *info, cudaStream_t st) {
+    static PerDevice<bool> smem_set;  // allow the largest size once per device
+    smem_set.get([] {
+        GCGE_CUDA(cudaFuncSetAttribute(k_jacobi_cta<IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)jacobi_cta_smem_bytes(kJacCtaMax)));
+        return true;
+    });
+    const int np = jac_m(s) / 2, threads = std::min(kJacobiThreads, (np * np + 31) / 32 * 32);
+    k_jacobi_cta<IT><<<1, threads, jacobi_cta_smem_bytes(s), st>>>(s, M, ldm, log, max_rounds,
+                                                                  info);
+    GCGE_CHECK_LAUNCH();
+}
+
 // ---------------------------------------------------------------- cluster Jacobi
 // The same rotations in a cluster of kJC CTAs.  Indices are arranged by the
 // circle method: with P_r[0] = 0 and P_r[i] = 1 + ((i - 1 - r) mod (m - 1)),
@@ -234,14 +391,11 @@ k_jacobi32(int s, const double *__restrict__ M, int ldm, float4 *__restrict__ lo
 //   (c) one cluster barrier makes the next buffers and tables complete.
 // The round is bound by the latency of its serial chain, of which a barrier is
 // the longest link: computing the rotations eight times over costs less than
-// the second barrier that sharing them took.
+// the second barrier that sharing them took (whole eigensolve of s = 180 1.55 ms
+// with two barriers, 1.43 with one).
 // The stopping test is that of k_jacobi32; every CTA sums the per-CTA
 // off-diagonal masses in the same order, so all take the same decision.
 constexpr int kJC = 8;
-// Smaller matrices use the one-CTA kernel.  Measured on GB300 (RR-shaped
-// matrices, kernel time): s = 64, 80: one CTA 480, 609 us, cluster 510, 652 us;
-// s = 96, 128, 200: one CTA 1152, 2321, 8161 us, cluster 956, 1290, 2403 us.
-constexpr int kJacClusterMin = 88;
 constexpr int kJacMaxLocal = 32;    // slots per CTA (np <= 256: s <= 512)
 
 __host__ __device__ inline int jc_slots(int np) { return (np + kJC - 1) / kJC; }
@@ -561,17 +715,17 @@ constexpr int kCircleAhead = 4;
 template <int NS>
 __global__ void __launch_bounds__(128)
 k_apply_circle(int s, const float2 *__restrict__ log, const int *__restrict__ info,
-               double *__restrict__ V, int ldv) {
+               double *__restrict__ V, int ldv, bool reversed) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int row = blockIdx.x * 4 + warp;
     if (row >= s) return;  // warp-uniform; the kernel has no block-wide barrier
     const int m = jac_m(s), np = m / 2, rounds = info[0];
-    const int k0 = lane * NS;
+    const int k0 = lane * NS, pos = reversed ? m - 1 - row : row;
     float top[NS], bot[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-        top[j] = k0 + j == row ? 1.0f : 0.0f;
-        bot[j] = m - 1 - (k0 + j) == row ? 1.0f : 0.0f;
+        top[j] = k0 + j == pos ? 1.0f : 0.0f;
+        bot[j] = m - 1 - (k0 + j) == pos ? 1.0f : 0.0f;
     }
     float2 q[kCircleAhead][NS];
     auto load = [&](float2 (&dst)[NS], int t) {
@@ -587,6 +741,7 @@ k_apply_circle(int s, const float2 *__restrict__ log, const int *__restrict__ in
             top[j] = e[j].x * vt - e[j].y * vb;
             bot[j] = e[j].y * vt + e[j].x * vb;
         }
+        if (NS == 1 && np == 1) return;  // a single pair stays where it is
         // top k -> top k + 1, bottom k -> bottom k - 1; top 0 stays, bottom 0 ->
         // top 1, top np - 1 -> bottom np - 1
         const float b0 = bot[0];
@@ -614,10 +769,10 @@ k_apply_circle(int s, const float2 *__restrict__ log, const int *__restrict__ in
     }
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-        const int k = k0 + j;
+        const int k = k0 + j, ct = reversed ? m - 1 - k : k, cb = m - 1 - ct;
         if (k < np) {
-            V[row + (size_t)k * ldv] = (double)top[j];
-            if (m - 1 - k < s) V[row + (size_t)(m - 1 - k) * ldv] = (double)bot[j];
+            if (ct < s) V[row + (size_t)ct * ldv] = (double)top[j];
+            if (cb < s) V[row + (size_t)cb * ldv] = (double)bot[j];
         }
     }
 }
@@ -655,7 +810,7 @@ static bool jacobi_cluster_usable() {
 
 static int jacobi_cluster_max_dim() {
     const size_t lim = jacobi_cluster_dyn_limit();
-    int s = kJacClusterMin;
+    int s = kJacCtaMax;
     while (jacobi_cluster_smem_bytes(s + 1) <= lim && jc_slots(jac_m(s + 1) / 2) <= kJacMaxLocal)
         ++s;
     return s;
@@ -775,34 +930,43 @@ int sym_eig(EigWork &wk, int s, const double *M, int ld, double *eval_host, doub
                                        (int)jacobi_dyn_limit()));
         return true;
     });
-    const bool cluster = s >= kJacClusterMin && jacobi_cluster_usable() &&
+    const bool cta = s <= kJacCtaMax;
+    const bool cluster = !cta && jacobi_cluster_usable() &&
                          jacobi_cluster_smem_bytes(s) <= jacobi_cluster_dyn_limit() &&
                          jc_slots(jac_m(s) / 2) <= kJacMaxLocal;
-    if (cluster) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kJC);
-        cfg.blockDim = dim3(kJacobiThreads);
-        cfg.dynamicSmemBytes = jacobi_cluster_smem_bytes(s);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kJC;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+    if (cluster || cta) {
         float2 *log = reinterpret_cast<float2 *>(wk.log.p);
-        GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi32_cluster, s, M, ld, log, wk.max_rounds,
-                                     wk.info.p));
-        GCGE_CHECK_LAUNCH();
+        if (cta) {
+            const int np = jac_m(s) / 2;
+            auto go = np <= 32   ? launch_jacobi_cta<1>
+                      : np <= 45 ? launch_jacobi_cta<2>
+                                 : launch_jacobi_cta<3>;  // 55^2 = 3025 blocks
+            go(s, M, ld, log, wk.max_rounds, wk.info.p, st);
+        } else {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(kJC);
+            cfg.blockDim = dim3(kJacobiThreads);
+            cfg.dynamicSmemBytes = jacobi_cluster_smem_bytes(s);
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = kJC;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            GCGE_CUDA(cudaLaunchKernelEx(&cfg, k_jacobi32_cluster, s, M, ld, log, wk.max_rounds,
+                                         wk.info.p));
+            GCGE_CHECK_LAUNCH();
+        }
         const int grid = (s + 3) / 4;
         switch ((jac_m(s) / 2 + 31) / 32) {
 #define GCGE_CIRCLE_CASE(NS)                                                        \
     case NS:                                                                        \
-        k_apply_circle<NS><<<grid, 128, 0, st>>>(s, log, wk.info.p, wk.X.p, s);      \
+        k_apply_circle<NS><<<grid, 128, 0, st>>>(s, log, wk.info.p, wk.X.p, s, cta); \
         break;
-            GCGE_CIRCLE_CASE(2) GCGE_CIRCLE_CASE(3) GCGE_CIRCLE_CASE(4) GCGE_CIRCLE_CASE(5)
-            GCGE_CIRCLE_CASE(6) GCGE_CIRCLE_CASE(7) GCGE_CIRCLE_CASE(8)
+            GCGE_CIRCLE_CASE(1) GCGE_CIRCLE_CASE(2) GCGE_CIRCLE_CASE(3) GCGE_CIRCLE_CASE(4)
+            GCGE_CIRCLE_CASE(5) GCGE_CIRCLE_CASE(6) GCGE_CIRCLE_CASE(7) GCGE_CIRCLE_CASE(8)
 #undef GCGE_CIRCLE_CASE
             default: throw CudaError{GCGE_ERR_TOO_LARGE, "sym_eig: size"};
         }
@@ -813,7 +977,6 @@ int sym_eig(EigWork &wk, int s, const double *M, int ld, double *eval_host, doub
                                                                     wk.max_rounds, wk.info.p);
         GCGE_CHECK_LAUNCH();
         switch ((jac_m(s) / 2 + 31) / 32) {
-            case 1: launch_rotations<1>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
             case 2: launch_rotations<2>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
             case 3: launch_rotations<3>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
             case 4: launch_rotations<4>(s, wk.log.p, wk.info.p, wk.X.p, s, st); break;
