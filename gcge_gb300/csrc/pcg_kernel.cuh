@@ -830,9 +830,11 @@ __device__ __forceinline__ bool grid_arrive_wait(PcgSync *gs, int *error,
 // alpha barrier.  Otherwise (FP64 operators with enough entries per row that
 // the gather's second FMA costs more than a barrier): p is stored first, and
 // gathered after a barrier of its own.  CL: the blocks are one thread-block
-// cluster and its hardware barrier replaces the grid's.
+// cluster, its hardware barrier replaces the grid's, and every block puts its
+// partial sums into the others' shared memory.
 //
 constexpr int kSmallThreads = 512;
+constexpr int kSmallCluster = 16;          // blocks of the cluster form at most
 constexpr int kSmallSmemMax = 160 * 1024;  // the rest stays L1
 // Element offset of row i, 16-byte group u of a slice-blocked block of G groups
 // (a small operator's blocks have fewer than 2^31 elements).
@@ -842,20 +844,22 @@ __device__ __forceinline__ unsigned goff(int i, int u, int G) {
     return (((unsigned)i >> 5) * (unsigned)G + (unsigned)u) * (32u * L) + ((unsigned)i & 31u) * L;
 }
 
-// acc += N entries (col[0], col[32], ..) of the lane's row times the groups
-// [u0, u0 + GU) of V, or with RP of V + beta Vp.  A group past the last one
-// repeats it; its sums are not used.
+// acc += N entries (col[0], col[32], ..) of the lane's row, of which `left` are
+// its own, times the groups [u0, u0 + GU) of V, or with RP of V + beta Vp.  An
+// entry past the last one repeats its loads only; a group past the last one
+// repeats it, and its sums are not used.
 template <typename T, int GU, int N, bool RP>
-__device__ __forceinline__ void unit_entries(const int *col, const T *val, const T *V, const T *Vp,
-                                             const T *beta, int u0, int G,
+__device__ __forceinline__ void unit_entries(const int *col, const T *val, int left, const T *V,
+                                             const T *Vp, const T *beta, int u0, int G,
                                              T (&acc)[GU * Pk<T>::L]) {
     constexpr int L = Pk<T>::L;
     int j[N];
     T m[N];
 #pragma unroll
     for (int d = 0; d < N; ++d) {
-        j[d] = col[32 * d];
-        m[d] = val[32 * d];
+        const int dd = min(d, left - 1);
+        j[d] = col[32 * dd];
+        m[d] = val[32 * dd];
     }
     Pk<T> q0[N][GU], q1[N][GU];
 #pragma unroll
@@ -869,6 +873,7 @@ __device__ __forceinline__ void unit_entries(const int *col, const T *val, const
     }
 #pragma unroll
     for (int d = 0; d < N; ++d) {
+        if (d >= left) continue;  // the same for the whole warp
 #pragma unroll
         for (int g = 0; g < GU; ++g) {
 #pragma unroll
@@ -891,13 +896,24 @@ __device__ __forceinline__ void unit_gather(const int *col, const T *val, int wi
         acc[c] = T(0);
         beta[c] = RP ? sbeta[c] : T(0);
     }
-    int e = 0;
 #pragma unroll 1
-    for (; e + NE <= width; e += NE)
-        unit_entries<T, GU, NE, RP>(col + 32 * e, val + 32 * e, V, Vp, beta, u0, G, acc);
-#pragma unroll 1
-    for (; e < width; ++e)
-        unit_entries<T, GU, 1, RP>(col + 32 * e, val + 32 * e, V, Vp, beta, u0, G, acc);
+    for (int e = 0; e < width; e += NE)
+        unit_entries<T, GU, NE, RP>(col + 32 * e, val + 32 * e, width - e, V, Vp, beta, u0, G, acc);
+}
+
+// a / b for a coefficient that is used in T.  For FP32 the reciprocal's FP32 value
+// and one Newton step in FP64, y + y (1 - b y): three dependent FP64 operations
+// instead of a division's chain, and a relative error below 2^-45.
+template <typename T>
+__device__ __forceinline__ double scalar_quotient(double a, double b) {
+    if constexpr (sizeof(T) == 4) {
+        const double m = fabs(b);
+        if (m > 1e-30 && m < 1e30) {
+            const double y = (double)(1.0f / (float)b);
+            return a * fma(y, fma(-b, y, 1.0), y);
+        }
+    }
+    return a / b;
 }
 
 template <typename T, int GU, int U, bool CL, bool FUSE>
@@ -905,11 +921,17 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
 k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     constexpr int L = Pk<T>::L, CC = GU * L;
     constexpr int NW = kSmallThreads / 32;
-    constexpr int NE = 8 / (U * GU * (FUSE ? 2 : 1));  // matrix entries in flight per lane
+    // matrix entries in flight per lane (a 5- or 7-point row in one go)
+    constexpr int NE = U * GU == 1 ? (sizeof(T) == 8 && FUSE ? 5 : 8)
+                       : U * GU == 4 && FUSE ? 1
+                                             : 8 / (U * GU * (FUSE ? 2 : 1));
     extern __shared__ __align__(16) unsigned char dsm[];
-    __shared__ double wred[NW * U][CC];  // column sums of each unit
+    __shared__ T wred[NW * U][CC];  // column sums of each unit
     __shared__ double sums[2][kPcgMaxCols];
-    __shared__ double stripe[kSmallThreads];
+    __shared__ double stop[kPcgMaxCols];  // r^T r at which a column leaves
+    // the partial sums of every block of the cluster, two sets of two; else the
+    // column sums of each stripe
+    __shared__ double stripe[CL ? 4 * kSmallCluster * kPcgMaxCols : kSmallThreads];
     __shared__ T s_alpha[kPcgMaxCols], s_beta[kPcgMaxCols];
     __shared__ int s_act[kPcgMaxCols];
     __shared__ int s_nactive;
@@ -922,6 +944,7 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     const int nb = gridDim.x, me = blockIdx.x;
     const bool stats_block = me == 0;
     if (!CL && a.withhold_last && nb > 1 && me == nb - 1) return;
+    if constexpr (CL) cooperative_groups::this_cluster().sync();  // all blocks run
 
     const int s0 = (int)((long long)a.nslices * me / nb);
     const int s1 = (int)((long long)a.nslices * (me + 1) / nb);
@@ -999,7 +1022,7 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     // column sums of q over the unit's rows, into its row of wred
     auto unit_sum = [&](int i, T (&q)[CC]) {
         const T s = warp_cols_reduce<T, CC>(q, lane);
-        if (lane < CC) wred[warp + i * NW][lane] = (double)s;
+        if (lane < CC) wred[warp + i * NW][lane] = s;
     };
     // Two sets of partials alternate by the barrier's parity: blocks read them
     // after a barrier while faster ones already write the next phase's, and a set
@@ -1008,41 +1031,69 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     auto part_of = [&](unsigned long long e, int which) {
         return a.part + ((size_t)(e & 1) * 2 + which) * nb * kp;
     };
-    // this block's column sums of wred, for the next barrier
+    // Column sums over `count` values get(b, c): Q lanes of a warp a column, each
+    // every Q-th value, then a tree over the lanes; use(c, sum, q) on all of
+    // them.  (An FP64 addition occupies a scheduler for 64 clocks whatever the
+    // lanes at work: a column's chain is kept short and few warps take part.)
+    const int Q = kp <= 16 ? 8 : 4;
+    auto col_sums = [&](int count, auto get, auto use) {
+        if (tid >= ((kp * Q + 31) & ~31)) return;
+        const int c = tid / Q, q = tid % Q;
+        double t = 0.0;
+        if (c < kp && q < count) {
+            t = get(q, c);
+            for (int b = q + Q; b < count; b += Q) t += get(b, c);
+        }
+        for (int o = Q / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (c < kp) use(c, t, q);
+    };
+    // this block's column sums of wred, for the next barrier: into the other
+    // blocks' shared memory in a cluster, else into global memory
     auto publish = [&](int which) {
         __syncthreads();
-        if (tid < kp) {
-            const int ch = tid / CC, c = tid % CC;
-            double s4[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int sl = 0; sl < nsl; ++sl) s4[sl & 3] += wred[sl * nch + ch][c];
-            part_of(epoch + 1, which)[(size_t)me * kp + tid] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        }
+        col_sums(
+            nsl, [&](int sl, int c) { return (double)wred[sl * nch + c / CC][c % CC]; },
+            [&](int c, double t, int q) {
+                if constexpr (CL) {
+                    double *at = stripe + ((((epoch + 1) & 1) * 2 + which) * nb + me) * kp + c;
+                    for (int b = q; b < nb; b += Q)
+                        *cooperative_groups::this_cluster().map_shared_rank(at, b) = t;
+                } else if (q == 0) {
+                    part_of(epoch + 1, which)[(size_t)me * kp + c] = t;
+                }
+            });
     };
-    // Sums of the partials over the blocks: `stripes` threads per column, each
-    // a fixed share of the blocks, then a fixed tree.
-    auto total = [&](int which, double *out) {
-        const double *part = part_of(epoch, which);
-        const int stripes = kSmallThreads / kp;
-        const int c = tid % kp, st = tid / kp;
-        double t0 = 0.0, t1 = 0.0;
-        if (st < stripes) {
-            int b = st;
-            for (; b + stripes < nb; b += 2 * stripes) {
-                t0 += __ldcg(part + (size_t)b * kp + c);
-                t1 += __ldcg(part + (size_t)(b + stripes) * kp + c);
+    // Sums of the partials over the blocks, used by lane 0 of each column's;
+    // the caller synchronises the block.  From global memory `stripes` threads a
+    // column first add a fixed share of the blocks each.
+    auto total = [&](int which, auto use) {
+        auto first = [&](int c, double t, int q) {
+            if (q == 0) use(c, t);
+        };
+        if constexpr (CL) {
+            const double *part = stripe + ((epoch & 1) * 2 + which) * nb * kp;
+            col_sums(nb, [&](int b, int c) { return part[b * kp + c]; }, first);
+        } else {
+            const double *part = part_of(epoch, which);
+            const int stripes = min(min(kSmallThreads / kp, 32), nb);
+            const int c = tid % kp, st = tid / kp;
+            if (st < stripes) {
+                double t0 = __ldcg(part + (size_t)st * kp + c);
+                double t1 = 0.0;
+                int b = st + stripes;
+                if (b < nb) t1 = __ldcg(part + (size_t)b * kp + c);
+                for (b += stripes; b + stripes < nb; b += 2 * stripes) {
+                    const double v0 = __ldcg(part + (size_t)b * kp + c);
+                    const double v1 = __ldcg(part + (size_t)(b + stripes) * kp + c);
+                    t0 += v0;
+                    t1 += v1;
+                }
+                if (b < nb) t0 += __ldcg(part + (size_t)b * kp + c);
+                stripe[tid] = t0 + t1;
             }
-            if (b < nb) t0 += __ldcg(part + (size_t)b * kp + c);
-        }
-        stripe[tid] = t0 + t1;
-        __syncthreads();
-        for (int wd = min(stripes, nb); wd > 1;) {
-            const int half = (wd + 1) / 2;
-            if (tid < (wd - half) * kp) stripe[tid] += stripe[tid + half * kp];
             __syncthreads();
-            wd = half;
+            col_sums(stripes, [&](int st, int c) { return stripe[st * kp + c]; }, first);
         }
-        if (tid < kp) out[tid] = stripe[tid];
-        __syncthreads();
     };
     auto barrier = [&]() {
         ++epoch;
@@ -1059,6 +1110,8 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
         for (int i = 0; i < U; ++i)
             if (live[i]) store(a.X, i, x[i]);
         if (me == 0) {  // the host reads the first block's scalars
+            if (tid < k) sc->last_res[tid] = sqrt(sc->rho2[tid]);
+            __syncthreads();
             const int *src = reinterpret_cast<const int *>(sc);
             int *dst = reinterpret_cast<int *>(a.sc);
             for (int i = tid; i < (int)(sizeof(PcgScalars) / sizeof(int)); i += kSmallThreads)
@@ -1116,8 +1169,12 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
         return;
     }
     // initial residual norms (src/ops_lin_sol.c:171-233)
-    total(0, sums[0]);
-    if (a.rel_tol) total(1, sums[1]);
+    total(0, [&](int c, double t) { sums[0][c] = t; });
+    if (a.rel_tol) {
+        __syncthreads();
+        total(1, [&](int c, double t) { sums[1][c] = t; });
+    }
+    __syncthreads();
     if (tid < kPcgMaxCols) {
         const int c = tid;
         int on = 0;
@@ -1131,6 +1188,8 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             sc->beta[c] = 0.0;
             sc->alpha[c] = 0.0;
             on = res > a.tol * nrm ? 1 : 0;
+            const double lim = fmax(a.rate * res, a.tol * nrm);
+            stop[c] = lim * lim;
         }
         sc->active[c] = s_act[c] = on;
         sc->left_at[c] = 0;
@@ -1193,17 +1252,16 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             return;
         }
         // alpha = rho / p^T w (src/ops_lin_sol.c:300-330)
-        total(0, sums[0]);
-        if (tid < k) {
-            const int c = tid;
-            const double ptw = sums[0][c], rho = sc->rho2[c];
-            const double al = s_act[c] ? rho / ptw : 0.0;
+        total(0, [&](int c, double ptw) {
+            if (c >= k) return;
+            const double rho = sc->rho2[c];
+            const double al = s_act[c] ? scalar_quotient<T>(rho, ptw) : 0.0;
             sc->ptw[c] = ptw;
             sc->rho1[c] = rho;
             sc->alpha[c] = al;
             s_alpha[c] = (T)al;
-        }
-        if (tid == 32 && stats_block) {
+        });
+        if (tid == kSmallThreads - 1 && stats_block) {
             int gact = 0;
             for (int u = 0; u < G; ++u) {
                 int any = 0;
@@ -1243,28 +1301,23 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             finish(false);
             return;
         }
-        // convergence test of src/ops_lin_sol.c:383-394 (threads 64 on) and beta
-        // for the next step
-        total(0, sums[0]);
-        if (tid < k && s_act[tid]) {
-            const double rr = sums[0][tid], be = rr / sc->rho1[tid];
-            sc->rho2[tid] = rr;
-            sc->beta[tid] = be;
-            s_beta[tid] = (T)be;
-        }
-        int leave = 0;
-        if (tid >= 64 && tid < 64 + k && s_act[tid - 64]) {
-            const int c = tid - 64;
-            const double res = sqrt(sums[0][c]);
-            sc->last_res[c] = res;
-            if (!(res > a.rate * sc->init_res[c] && res > a.tol * sc->norm_b[c])) {
+        // convergence test of src/ops_lin_sol.c:383-394, on squares, and beta for
+        // the next step
+        int leave = -1;
+        total(0, [&](int c, double rr) {
+            if (c >= k || !s_act[c]) return;
+            const double be = scalar_quotient<T>(rr, sc->rho1[c]);
+            sc->rho2[c] = rr;
+            sc->beta[c] = be;
+            s_beta[c] = (T)be;
+            if (!(rr > stop[c])) {
                 sc->active[c] = 0;
                 sc->left_at[c] = it + 1;
-                leave = 1;
+                leave = c;
             }
-        }
-        const int left = __syncthreads_count(leave);
-        if (leave) s_act[tid - 64] = 0;
+        });
+        const int left = __syncthreads_count(leave >= 0);
+        if (leave >= 0) s_act[leave] = 0;
         if (tid == 0) {
             s_nactive -= left;
             sc->nactive = s_nactive;
@@ -1287,7 +1340,7 @@ int pcg_small_cluster() {
             cudaGetLastError();
             return 0;
         }
-        for (int c : {16, 8}) {
+        for (int c : {kSmallCluster, 8}) {
             if (c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed,
                                               1) != cudaSuccess) {
                 cudaGetLastError();
@@ -1352,24 +1405,33 @@ void launch_pcg_small_form(const PcgArgs<T> &a, int kp, bool cluster, int nb, cu
 
 // Runs the solve in k_pcg_small where the units of its operator fit the warps
 // (two each); false where they do not, and the three-phase grid kernel takes it.
-// Measured, us per step, three-phase kernel (or its former cluster form) ->
-// this one:
-//   5-point n = 4160    k = 4 FP32 9.3 -> 7.7, FP64 16 -> 11.8; k = 20 FP64 37 -> 13.6
-//   5-point n = 16384   k = 4 FP32 13 -> 10.7, FP64 24 -> 12.4; k = 20 27 -> 12.8, 38 -> 22.8
-//   7-point 32^3        k = 4 FP32 22 -> 11.8, FP64 26 -> 15.4; k = 20 FP32 29 -> 17.0
-//   27-point 24^3       k = 20 FP32 36 -> 15.1, FP64 59 -> 29.5; 40^3 k = 12 FP32 32 -> 22.5
+// Measured, us per step of a 30-step solve, three-phase kernel (or its former
+// cluster form) -> this one:
+//   5-point n = 4160    k = 4 FP32 9.3 -> 4.6, FP64 16 -> 8.8; k = 20 FP64 37 -> 11.9
+//   5-point n = 16384   k = 4 FP32 13 -> 7.8, FP64 24 -> 9.7; k = 20 27 -> 10.5, 38 -> 21.1
+//   7-point 32^3        k = 4 FP32 22 -> 8.4, FP64 26 -> 13.0; k = 20 FP32 29 -> 15.2
+//   27-point 24^3       k = 20 FP32 36 -> 13.3, FP64 59 -> 28.3
+// Most of a short step is not the gather but the FP64 scalars: with a block-wide
+// tree over every block's partials, a division and a square root a step took
+// 7.3 us at n = 4160, k = 4 FP32 (7.3 -> 4.6; n = 16384 10.3 -> 7.8; 27-point 24^3,
+// k = 20 14.7 -> 13.3).
 // FUSE: the gather's second vector against a barrier.  In FP64 its FMAs decide
 // (entries k / 2 clocks over the SMs; 5-point k = 20, n = 7400: 16.8 us both at
 // 2429, k = 12 14.1 against 14.8 at 1458, k = 40 26.2 against 24.5 at 4859), in
 // FP32 its loads (27-point 24^3, k = 20 15.1 against 15.3 at 23900, k = 40 20.0
 // against 18.4 at 47700).
-// Cluster or grid: the cluster's barriers are shorter, but it has 16 of the 152
-// SMs (FP32 n = 4160: k = 4 7.7 against 10.5 us, k = 12 10.5 against 11.1, k = 20
-// 11.9 against 11.6; FP64 k = 4 11.8 both).
+// Cluster or grid: the cluster's barriers are shorter and its partials stay in
+// shared memory, but it has 16 of the 152 SMs.  FP32, cluster against grid: with
+// a unit per warp 5-point n = 7400, k = 8 (2300 clocks) 6.1 against 8.1 us, 7-point
+// 20^3, k = 8 (3500) 6.7 against 8.0; with two, n = 4160, k = 12 (1950) 7.7
+// against 8.3, n = 16384, k = 4 (2560) 8.8 against 7.8, n = 7400, k = 12 (3470) 8.9
+// against 8.7.  FP64 n = 4160, k = 4 (7800) 9.6 against 8.8.
 template <typename T>
 constexpr double kFuseClocks = sizeof(T) == 8 ? 2200.0 : 30000.0;
 template <typename T>
-constexpr double kClusterClocks = sizeof(T) == 8 ? 6000.0 : 2000.0;
+constexpr double cluster_clocks(bool one_unit) {
+    return sizeof(T) == 8 ? 6000.0 : one_unit ? 4000.0 : 2000.0;
+}
 template <typename T>
 bool launch_pcg_small(const PcgArgs<T> &a, int kp, cudaStream_t st) {
     constexpr int NW = kSmallThreads / 32;
@@ -1385,7 +1447,8 @@ bool launch_pcg_small(const PcgArgs<T> &a, int kp, cudaStream_t st) {
     const int csize = std::min(pcg_small_cluster<T, 1, 1>(),
                                std::min(pcg_small_cluster<T, 2, 1>(), pcg_small_cluster<T, 2, 2>()));
     const bool cluster =
-        fuse && csize > 0 && units(csize, 2) <= 2 * NW && work / csize <= kClusterClocks<T>;
+        fuse && csize > 0 && units(csize, 2) <= 2 * NW &&
+        work / csize <= cluster_clocks<T>(units(csize, 2) <= NW);
     const int nb = cluster ? csize : std::max(1, std::min(sms, a.nslices));
     if (!cluster && units(nb, 2) > 2 * NW) return false;
     // narrow chunks while every warp has one unit at most: more warps at work

@@ -121,3 +121,15 @@ def test_relative_tolerance_through_the_linear_solver_hook(gpu_lib):
     ref = x0.copy(order="F")
     GCGOracle(A.to_scipy(), None, p).block_pcg(np.asfortranarray(b), ref)
     assert np.linalg.norm(x - ref) / np.linalg.norm(ref) < 3.3e-12
+
+
+@pytest.mark.parametrize("nx,ny,k", [(100, 74, 8), (100, 74, 12), (100, 75, 7), (64, 65, 20)])
+def test_cluster_and_grid_forms_in_fp32(gpu_lib, nx, ny, k):
+    """Either side of the cluster form's rule: one and two units a warp."""
+    A = shifted(P.laplace2d(nx, ny), 0.1)
+    b = columns(A.n, k, nx + k).astype(np.float32).astype(np.float64)
+    x0 = np.zeros_like(b)
+    ref, it_ref = oracle(A, b, x0, 1e-4)
+    x, it = gpu_lib.block_pcg(A, None, 0.0, b, x0, max_iter=30, rate=1e-4, tol=1e-14, fp32=True)
+    assert np.linalg.norm(x - ref) / np.linalg.norm(ref) < 1.8e-3
+    assert abs(it - it_ref) <= 1
