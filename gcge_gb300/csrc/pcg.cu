@@ -108,7 +108,7 @@ PcgWork::~PcgWork() {
 void PcgWork::reserve(int n, int kmax_) {
     (void)n;
     kmax = std::max(kmax_, 40);
-    part.alloc((size_t)2 * kMaxBlocksPerSm * device_sms() * kPcgMaxCols);
+    part.alloc((size_t)4 * device_sms() * kPcgMaxCols);
     if (!sc.p) {
         sc.alloc(1);
         sync.alloc(1);

@@ -23,10 +23,8 @@ struct PcgScalars {
 // Grid barrier state of the persistent solve kernel (zeroed before each
 // launch) and counters that accumulate over launches.
 struct PcgSync {
-    unsigned long long arrive;   // block arrivals at barriers, over the launch
-    unsigned long long release;  // number of the last barrier released
-    unsigned long long t_spmm;   // globaltimer at the start of the SpMM phase
-    int error;                   // a barrier wait ran out of time
+    unsigned long long arrive;  // block arrivals at barriers, over the launch
+    int error;                  // a barrier wait ran out of time
     int pad;
 };
 struct PcgStats {

@@ -8,17 +8,19 @@
 // barriers:
 //   1. p = r + beta p                      (own rows; p = r on the first step)
 //   2. w = S p, partial sums of p^T w      (warp per slice, gathers p rows)
-//      -> the last block to arrive sums the partials: alpha = rho / p^T w
+//      -> every block sums the blocks' partials: alpha = rho / p^T w
 //   3. x += alpha p, r -= alpha w, partial sums of r^T r
-//      -> the last block: residual norms, convergence test, beta, count
+//      -> residual norms, convergence test, beta, count
 // so nothing returns to the host between iterations.  The reference keeps a
 // compacted list of unconverged columns and runs one SpMM per contiguous run
 // of them; here a per-column `active` flag plays that role: inactive columns
 // keep x and r (alpha = 0), drop out of the sums, and a 16-byte group of
 // columns that is wholly inactive is neither gathered nor updated.
 //
-// Cross-block sums are taken by one block in a fixed order, so results are
-// deterministic for a given grid.  The shifted operator is one SELL matrix
+// Every block takes the cross-block sums for itself, all in the same fixed order,
+// so results are deterministic for a given grid.  (With two blocks an SM, the
+// last of them to arrive summing for all and the scalars in global memory, the
+// barriers took 20 us of a step of 92 at 64^3 with 27 points and 20 columns.)  The shifted operator is one SELL matrix
 // S = A + sigma B on the union pattern of A and B (the reference's in-place
 // MatAxpby branch, src/ops_eig_sol_gcg.c:600-608), so each iteration streams
 // one matrix.  Vectors are slice-blocked n x kp blocks (kp = k padded to 16
@@ -175,53 +177,37 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
 
-// Grid-wide barrier number `epoch` (1, 2, ...).  The last block to arrive runs
-// `last` with all its threads before it releases the others, so the
-// cross-block reductions are done once.  Returns false when the wait ran out
-// (or another block's did); the caller then returns.
-template <typename F>
-__device__ __forceinline__ bool grid_sync(PcgSync *gs, int *error, unsigned long long timeout_ns,
-                                          long long max_polls, unsigned long long epoch,
-                                          F &&last) {
-    __shared__ int s_last, s_ok;
+// Grid-wide barrier number `epoch` (1, 2, ...): every block waits for the
+// arrivals of all.  Returns false when the wait ran out (or another block's
+// did); the caller then returns.
+__device__ __forceinline__ bool grid_arrive_wait(PcgSync *gs, int *error,
+                                                 unsigned long long timeout_ns,
+                                                 long long max_polls, unsigned long long epoch) {
+    __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned long long old = atomicAdd(&gs->arrive, 1ull);
-        const int lst = old + 1ull == epoch * gridDim.x;
-        if (lst) __threadfence();
-        s_last = lst;
         s_ok = 1;
-    }
-    __syncthreads();
-    if (s_last) {
-        last();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            st_release(&gs->release, epoch);
-        }
-    } else if (threadIdx.x == 0) {
-        const unsigned long long t0 = global_ns();
-        for (long long poll = 0; ld_acquire(&gs->release) < epoch; ++poll) {
-            if ((poll & 31) == 31 &&
-                (*(volatile int *)error != 0 || poll > max_polls ||
-                 global_ns() - t0 > timeout_ns)) {
-                atomicExch(error, 1);
-                s_ok = 0;
-                break;
+        __threadfence();
+        const unsigned long long all = epoch * gridDim.x;
+        if (atomicAdd(&gs->arrive, 1ull) + 1ull < all) {
+            const unsigned long long t0 = global_ns();
+            for (long long poll = 0; ld_acquire(&gs->arrive) < all; ++poll) {
+                if ((poll & 31) == 31 &&
+                    (*(volatile int *)error != 0 || poll > max_polls ||
+                     global_ns() - t0 > timeout_ns)) {
+                    atomicExch(error, 1);
+                    s_ok = 0;
+                    break;
+                }
             }
-            __nanosleep(32);
         }
+        __threadfence();
     }
     __syncthreads();
     return s_ok != 0;
@@ -242,13 +228,39 @@ struct PcgArgs {
     PcgScalars *sc;
     PcgSync *sync;
     PcgStats *stats;
-    double *part;  // 2 x gridDim.x x KP
+    double *part;  // two sets (by barrier parity) of 2 x gridDim.x x kp
     // bound of every grid-barrier wait (device clock and poll count)
     unsigned long long timeout_ns;
     long long max_polls;
     // failure-detection test only: the grid's last block returns before its
     // first barrier, so the others' waits run out (never set otherwise)
     int withhold_last;
+};
+
+// What a launch adds to PcgStats, kept in shared memory by one thread until the
+// launch ends.
+template <typename T>
+struct PcgTally {
+    unsigned long long t0, ns;
+    long long groups;  // active 16-byte column groups, summed over the steps
+    int steps;
+    __device__ void clear() { ns = 0, groups = 0, steps = 0; }
+    __device__ void begin() { t0 = global_ns(); }
+    __device__ void end(int active_groups) {
+        ns += global_ns() - t0;
+        groups += active_groups;
+        ++steps;
+    }
+    __device__ void write(const PcgArgs<T> &a, int kp) const {
+        const double vec = (double)a.n * 16.0 * groups, start = 4.0 * a.n * kp * sizeof(T);
+        a.stats->spmm_ns += ns;
+        // SpMM: the matrix once, p read once, w written once
+        a.stats->spmm_bytes += steps * a.matrix_bytes + 2.0 * vec;
+        // step: p update (r, p read; p written), SpMM (p gathered and re-read, w
+        // written), x and r update (x, p, r, w read; x, r written)
+        a.stats->kernel_bytes +=
+            (a.x_zero ? 0.0 : a.matrix_bytes) + start + steps * a.matrix_bytes + 12.0 * vec;
+    }
 };
 
 // Compiler-only ordering point between the 16-byte groups of a row in the
@@ -307,59 +319,67 @@ __device__ __forceinline__ void warp_cols_add(const T (&acc)[KP], double *wrow, 
     }
 }
 
-// Column sums of the gridDim.x block partials part[b * KP + c] into
-// out[0..KP) (shared memory), fixed order: thread t adds blocks t / KP,
-// t / KP + S, ... of column t % KP (S = threads / KP stripes), then the
-// stripes are added pairwise in a fixed tree.
-template <int KP, int NT>
-__device__ __forceinline__ void grid_cols_sum(const double *part, double *out, double *stripe) {
-    constexpr int S = NT / KP;
-    const int t = threadIdx.x;
-    if (gridDim.x <= 32) {
-        // few blocks: one thread per column, four chains in a fixed order, no
-        // tree and its barriers
-        if (t < KP) {
-            const int nb = gridDim.x;
-            double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            int b = 0;
-            for (; b + 3 < nb; b += 4) {
-                s0 += __ldcg(part + (size_t)b * KP + t);
-                s1 += __ldcg(part + (size_t)(b + 1) * KP + t);
-                s2 += __ldcg(part + (size_t)(b + 2) * KP + t);
-                s3 += __ldcg(part + (size_t)(b + 3) * KP + t);
-            }
-            for (; b < nb; ++b) s0 += __ldcg(part + (size_t)b * KP + t);
-            out[t] = (s0 + s1) + (s2 + s3);
+// Column sums over `count` values get(b, c): Q lanes of a warp a column, each every
+// Q-th value, then a tree over the lanes; use(c, sum, q) on all of them.  (An
+// FP64 addition occupies a scheduler for 64 clocks whatever the lanes at work:
+// a column's chain is kept short and few warps take part.)
+template <typename Get, typename Use>
+__device__ __forceinline__ void lane_cols_sum(int kp, int count, Get get, Use use) {
+    const int tid = threadIdx.x, Q = kp <= 16 ? 8 : 4;
+    if (tid >= ((kp * Q + 31) & ~31)) return;
+    const int c = tid / Q, q = tid % Q;
+    double t = 0.0;
+    if (c < kp && q < count) {
+        t = get(q, c);
+        for (int b = q + Q; b < count; b += Q) t += get(b, c);
+    }
+    for (int o = Q / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (c < kp) use(c, t, q);
+}
+
+// Sums of the columns of the nb block partials part[b * kp + c], taken by every
+// block for itself; use(c, sum) on one lane each, and the caller synchronises the
+// block.  `stripes` threads a column first add a fixed share of the blocks.
+template <int NT, typename Use>
+__device__ __forceinline__ void grid_cols_sum(const double *part, int nb, int kp, double *stripe,
+                                              Use use) {
+    const int stripes = min(min(NT / kp, 32), nb);
+    const int c = threadIdx.x % kp, st = threadIdx.x / kp;
+    if (st < stripes) {  // L2 loads: other blocks wrote them
+        double t0 = __ldcg(part + (size_t)st * kp + c);
+        double t1 = 0.0;
+        int b = st + stripes;
+        if (b < nb) t1 = __ldcg(part + (size_t)b * kp + c);
+        for (b += stripes; b + stripes < nb; b += 2 * stripes) {
+            const double v0 = __ldcg(part + (size_t)b * kp + c);
+            const double v1 = __ldcg(part + (size_t)(b + stripes) * kp + c);
+            t0 += v0;
+            t1 += v1;
         }
-        __syncthreads();
-        return;
+        if (b < nb) t0 += __ldcg(part + (size_t)b * kp + c);
+        stripe[threadIdx.x] = t0 + t1;
     }
-    double s = 0.0;
-    if (t < S * KP) {
-        const int c = t % KP;
-        const int nb = gridDim.x;
-        int b = t / KP;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-        // L2 loads: the partials were written by other blocks on other SMs
-        for (; b + 3 * S < nb; b += 4 * S) {
-            s0 += __ldcg(part + (size_t)b * KP + c);
-            s1 += __ldcg(part + (size_t)(b + S) * KP + c);
-            s2 += __ldcg(part + (size_t)(b + 2 * S) * KP + c);
-            s3 += __ldcg(part + (size_t)(b + 3 * S) * KP + c);
+    __syncthreads();
+    lane_cols_sum(
+        kp, stripes, [&](int i, int col) { return stripe[i * kp + col]; },
+        [&](int col, double t, int q) {
+            if (q == 0) use(col, t);
+        });
+}
+
+// a / b for a coefficient that is used in T.  For FP32 the reciprocal's FP32 value
+// and one Newton step in FP64, y + y (1 - b y): three dependent FP64 operations
+// instead of a division's chain, and a relative error below 2^-45.
+template <typename T>
+__device__ __forceinline__ double scalar_quotient(double a, double b) {
+    if constexpr (sizeof(T) == 4) {
+        const double m = fabs(b);
+        if (m > 1e-30 && m < 1e30) {
+            const double y = (double)(1.0f / (float)b);
+            return a * fma(y, fma(-b, y, 1.0), y);
         }
-        for (; b < nb; b += S) s0 += __ldcg(part + (size_t)b * KP + c);
-        s = (s0 + s1) + (s2 + s3);
     }
-    stripe[t] = s;
-    __syncthreads();
-    for (int width = S; width > 1;) {
-        const int half = (width + 1) / 2;
-        if (t < (width - half) * KP) stripe[t] += stripe[t + half * KP];
-        __syncthreads();
-        width = half;
-    }
-    if (t < KP) out[t] = stripe[t];
-    __syncthreads();
+    return a / b;
 }
 
 // Wide blocks (at least 8 column groups, an even number) gather the SpMM
@@ -367,24 +387,19 @@ __device__ __forceinline__ void grid_cols_sum(const double *part, double *out, d
 template <typename T, int KP>
 constexpr bool kSplitGather = (KP / Pk<T>::L) >= 8 && (KP / Pk<T>::L) % 2 == 0;
 
-// Block shape by row width: 512 threads (two resident blocks, <= 64
-// registers) for rows up to 80 bytes and for FP32 rows of 40 columns (whose
-// phases run in two column parts: 4.76 -> 4.34 s of inner solve per 128^3
-// solve against one block per SM), 512 threads (<= 128 registers) up to 160
-// bytes, and 256 threads (<= 255 registers) for wider FP64 rows.
+// Block shape by row width, one block per SM: 1024 threads (<= 64 registers) for
+// rows up to 80 bytes and for FP32 rows of 40 columns (whose phases run in two
+// column parts: twice the warps hiding gather latency of 512 threads), 512
+// threads up to 160 bytes, and 256 threads for wider FP64 rows.
 template <typename T, int KP>
 __host__ __device__ constexpr int pcg_threads() {
-    return sizeof(T) * KP <= 160 ? 512 : 256;
-}
-template <typename T, int KP>
-__host__ __device__ constexpr int pcg_min_blocks() {
-    // FP32 rows of 40 columns fit 64 registers with their phases split into
-    // column parts: two blocks per SM, twice the warps hiding gather latency
-    return (sizeof(T) * KP <= 80 || (sizeof(T) == 4 && KP == 40)) ? 2 : 1;
+    return sizeof(T) * KP <= 80 || (sizeof(T) == 4 && KP == 40) ? 1024
+           : sizeof(T) * KP <= 160                              ? 512
+                                                                : 256;
 }
 
 template <typename T, int KP>
-__global__ void __launch_bounds__(pcg_threads<T, KP>(), pcg_min_blocks<T, KP>())
+__global__ void __launch_bounds__(pcg_threads<T, KP>(), 1)
 k_block_pcg(PcgArgs<T> a) {
     constexpr int kPcgThreads = pcg_threads<T, KP>();
     constexpr int L = Pk<T>::L;
@@ -399,35 +414,51 @@ k_block_pcg(PcgArgs<T> a) {
     };
     __shared__ double wred[nwarps][KP];  // per-warp column sums of one phase
     __shared__ double stripe[kPcgThreads];
-    __shared__ double sum1[KP], sum2[KP];
+    __shared__ double sums[2][KP];
+    __shared__ double stop[KP];  // r^T r at which a column leaves
+    __shared__ PcgScalars s_sc;  // every block's own, all the same
     __shared__ T s_coef[KP];
     __shared__ int s_act[KP];
     __shared__ int s_gact[G];
     __shared__ int s_nactive;
     __shared__ long long s_range[2];
 
-    PcgScalars *sc = a.sc;
+    PcgScalars *sc = &s_sc;
     PcgSync *gs = a.sync;
     int *error = &a.sync->error;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k = a.k, n = a.n;
-    const double vb = (double)sizeof(T);
     if (a.withhold_last && gridDim.x > 1 && blockIdx.x == gridDim.x - 1) return;
 
-    // per-warp accumulators: clear, and flush (fixed-order sum over warps)
+    const bool stats_thread = blockIdx.x == 0 && tid == kPcgThreads - 1;
+    __shared__ PcgTally<T> tally;
+    if (stats_thread) tally.clear();
+    const int nb = gridDim.x;
+    unsigned long long epoch = 0;
+    // Two sets of partials alternate by the barrier's parity: blocks read them
+    // after a barrier while faster ones already write the next phase's.
+    auto part_of = [&](unsigned long long e, int which) {
+        return a.part + ((size_t)(e & 1) * 2 + which) * nb * KP;
+    };
+    // per-warp accumulators: clear, and this block's sums for the next barrier
     auto wred_zero = [&]() {
         for (int i = tid; i < nwarps * KP; i += kPcgThreads) (&wred[0][0])[i] = 0.0;
         __syncthreads();
     };
-    auto wred_flush = [&](double *out) {
+    auto publish = [&](int which) {
         __syncthreads();
-        if (tid < KP) {
-            double s4[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-            for (int w = 0; w < nwarps; ++w) s4[w & 3] += wred[w][tid];
-            out[tid] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        }
+        lane_cols_sum(
+            KP, nwarps, [&](int w, int c) { return wred[w][c]; },
+            [&](int c, double t, int q) {
+                if (q == 0) part_of(epoch + 1, which)[(size_t)blockIdx.x * KP + c] = t;
+            });
         __syncthreads();
+    };
+    auto total = [&](int which, auto use) {
+        grid_cols_sum<kPcgThreads>(part_of(epoch, which), nb, KP, stripe, use);
+    };
+    auto barrier = [&]() {
+        return grid_arrive_wait(gs, error, a.timeout_ns, a.max_polls, ++epoch);
     };
 
     // slice range of this block, balanced by stored entries
@@ -445,16 +476,22 @@ k_block_pcg(PcgArgs<T> a) {
     __syncthreads();
     const int s0 = (int)s_range[0], s1 = (int)s_range[1];
     const int r0 = min(n, 32 * s0), r1 = min(n, 32 * s1);
-    unsigned long long epoch = 0;
-    // this block's partial sums, and of a second set (norms of b)
-    double *part1 = a.part + (size_t)blockIdx.x * KP;
-    double *part2 = a.part + (size_t)(gridDim.x + blockIdx.x) * KP;
 
     auto finish = [&](bool ok) {
-        if (blockIdx.x == 0 && tid == 0) {
-            if (!ok || *(volatile int *)error) a.stats->error = 1;
-            a.stats->launches += 1;
-            a.stats->iters += (unsigned long long)sc->niter;
+        __syncthreads();
+        if (blockIdx.x == 0) {  // the host reads the first block's scalars
+            if (tid < k) sc->last_res[tid] = sqrt(sc->rho2[tid]);
+            __syncthreads();
+            const int *src = reinterpret_cast<const int *>(sc);
+            int *dst = reinterpret_cast<int *>(a.sc);
+            for (int i = tid; i < (int)(sizeof(PcgScalars) / sizeof(int)); i += kPcgThreads)
+                dst[i] = src[i];
+            if (tid == 0) {
+                if (!ok || *(volatile int *)error) a.stats->error = 1;
+                a.stats->launches += 1;
+                a.stats->iters += (unsigned long long)sc->niter;
+            }
+            if (stats_thread) tally.write(a, KP);
         }
     };
 
@@ -521,7 +558,7 @@ k_block_pcg(PcgArgs<T> a) {
             });
         }
     }
-    wred_flush(part1);
+    publish(0);
     if (a.rel_tol) {
         wred_zero();
         for_parts([&](auto part) {
@@ -541,54 +578,53 @@ k_block_pcg(PcgArgs<T> a) {
             }
             warp_cols_add<T, KPP>(bacc, wred[warp] + U0 * L, lane);
         });
-        wred_flush(part2);
+        publish(1);
     }
-    // initial residual norms (src/ops_lin_sol.c:171-233)
-    if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
-            grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
-            if (a.rel_tol)
-                grid_cols_sum<KP, kPcgThreads>(a.part + (size_t)gridDim.x * KP, sum2, stripe);
-            if (tid < kPcgMaxCols) {
-                const int c = tid;
-                if (c < k) {
-                    const double nb = a.rel_tol ? sqrt(sum2[c]) : 1.0;
-                    const double rr = sum1[c];
-                    sc->norm_b[c] = nb;
-                    sc->rho2[c] = rr;
-                    sc->init_res[c] = sqrt(rr);
-                    sc->last_res[c] = sqrt(rr);
-                    sc->active[c] = sqrt(rr) > a.tol * nb ? 1 : 0;
-                    sc->left_at[c] = 0;
-                    sc->beta[c] = 0.0;
-                    sc->alpha[c] = 0.0;
-                } else {
-                    sc->active[c] = 0;
-                    sc->left_at[c] = 0;
-                }
-            }
-            __syncthreads();
-            if (tid == 0) {
-                int cnt = 0;
-                for (int c = 0; c < k; ++c) cnt += sc->active[c];
-                sc->nactive = cnt;
-                sc->niter = 0;
-                a.stats->kernel_bytes +=
-                    a.x_zero ? 4.0 * n * KP * vb : a.matrix_bytes + 4.0 * n * KP * vb;
-            }
-        })) {
+    if (!barrier()) {
+        if (tid == 0) sc->niter = 0;
         finish(false);
         return;
     }
-
-    for (int it = 0; it < a.max_iter; ++it) {
-        // ---------------- phase 1: p = r + beta p
-        if (tid < KP) {
-            s_act[tid] = sc->active[tid];
-            s_coef[tid] = (T)sc->beta[tid];
-        }
-        if (tid == 0) s_nactive = sc->nactive;
+    // initial residual norms (src/ops_lin_sol.c:171-233)
+    total(0, [&](int c, double v) { sums[0][c] = v; });
+    if (a.rel_tol) {
         __syncthreads();
-        if (s_nactive == 0) break;
+        total(1, [&](int c, double v) { sums[1][c] = v; });
+    }
+    __syncthreads();
+    if (tid < kPcgMaxCols) {
+        const int c = tid;
+        int on = 0;
+        if (c < k) {
+            const double nrm = a.rel_tol ? sqrt(sums[1][c]) : 1.0;
+            const double rr = sums[0][c], res = sqrt(rr);
+            sc->norm_b[c] = nrm;
+            sc->rho2[c] = rr;
+            sc->init_res[c] = res;
+            sc->last_res[c] = res;
+            sc->alpha[c] = sc->beta[c] = 0.0;
+            on = res > a.tol * nrm ? 1 : 0;
+            const double lim = fmax(a.rate * res, a.tol * nrm);
+            stop[c] = lim * lim;
+        }
+        sc->active[c] = on;
+        sc->left_at[c] = 0;
+        if (c < KP) {
+            s_act[c] = on;
+            s_coef[c] = T(0);  // beta of the first step
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        int cnt = 0;
+        for (int c = 0; c < k; ++c) cnt += s_act[c];
+        s_nactive = sc->nactive = cnt;
+        sc->niter = 0;
+    }
+    __syncthreads();
+
+    for (int it = 0; it < a.max_iter && s_nactive > 0; ++it) {
+        // ---------------- phase 1: p = r + beta p
         if (tid < G) {
             int any = 0;
             for (int q = 0; q < L; ++q) any |= s_act[tid * L + q];
@@ -611,12 +647,11 @@ k_block_pcg(PcgArgs<T> a) {
             }
         }
         wred_zero();
-        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
-                if (tid == 0) a.sync->t_spmm = global_ns();
-            })) {
+        if (!barrier()) {
             finish(false);
             return;
         }
+        if (stats_thread) tally.begin();
 
         // ---------------- phase 2: w = S p, p^T w
         {
@@ -689,38 +724,33 @@ k_block_pcg(PcgArgs<T> a) {
                     warp_cols_add<T, KP>(acc, wred[warp], lane);
                 }
             }
-            wred_flush(part1);
+            publish(0);
         }
-        // alpha = rho / p^T w (src/ops_lin_sol.c:300-330)
-        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
-                grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
-                if (tid < k) {
-                    const int c = tid;
-                    const double ptw = sum1[c];
-                    sc->ptw[c] = ptw;
-                    sc->rho1[c] = sc->rho2[c];
-                    sc->alpha[c] = sc->active[c] ? sc->rho2[c] / ptw : 0.0;
-                }
-                if (tid == 0) {
-                    int gact = 0;
-                    for (int u = 0; u < G; ++u) gact += s_gact[u];
-                    const double vec = (double)n * gact * L * vb;
-                    a.stats->spmm_ns += global_ns() - a.sync->t_spmm;
-                    // SpMM: the matrix once, p read once, w written once
-                    a.stats->spmm_bytes += a.matrix_bytes + 2.0 * vec;
-                    // iteration: phase 1 (r, p read; p written), phase 2 (p
-                    // gathered and re-read, w written), phase 3 (x, p, r, w
-                    // read; x, r written)
-                    a.stats->kernel_bytes += a.matrix_bytes + 12.0 * vec;
-                }
-            })) {
+        if (!barrier()) {
             finish(false);
             return;
         }
+        // alpha = rho / p^T w (src/ops_lin_sol.c:300-330)
+        total(0, [&](int c, double ptw) {
+            if (c >= k) {
+                s_coef[c] = T(0);
+                return;
+            }
+            const double rho = sc->rho2[c];
+            const double al = s_act[c] ? scalar_quotient<T>(rho, ptw) : 0.0;
+            sc->ptw[c] = ptw;
+            sc->rho1[c] = rho;
+            sc->alpha[c] = al;
+            s_coef[c] = (T)al;
+        });
+        if (stats_thread) {
+            int gact = 0;
+            for (int u = 0; u < G; ++u) gact += s_gact[u];
+            tally.end(gact);
+        }
 
         // ---------------- phase 3: x += alpha p, r -= alpha w, r^T r
-        if (tid < KP) s_coef[tid] = (T)sc->alpha[tid];
-        wred_zero();
+        wred_zero();  // (synchronises the block)
         for_parts([&](auto part) {
             constexpr int U0 = decltype(part)::value * GP;
             T racc[KPP];
@@ -752,67 +782,39 @@ k_block_pcg(PcgArgs<T> a) {
             }
             warp_cols_add<T, KPP>(racc, wred[warp] + U0 * L, lane);
         });
-        wred_flush(part1);
-        // convergence test of src/ops_lin_sol.c:383-394 and beta for the next step
-        if (!grid_sync(gs, error, a.timeout_ns, a.max_polls, ++epoch, [&]() {
-                grid_cols_sum<KP, kPcgThreads>(a.part, sum1, stripe);
-                if (tid < k && sc->active[tid]) {
-                    const int c = tid;
-                    const double rr = sum1[c];
-                    sc->rho2[c] = rr;
-                    const double res = sqrt(rr);
-                    sc->last_res[c] = res;
-                    sc->beta[c] = rr / sc->rho1[c];
-                    if (!(res > a.rate * sc->init_res[c] && res > a.tol * sc->norm_b[c])) {
-                        sc->active[c] = 0;
-                        sc->left_at[c] = sc->niter + 1;  // niter moves on after the barrier
-                    }
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    int cnt = 0;
-                    for (int c = 0; c < k; ++c) cnt += sc->active[c];
-                    sc->nactive = cnt;
-                    sc->niter += 1;
-                }
-            })) {
+        publish(0);
+        if (!barrier()) {
             finish(false);
             return;
         }
+        // convergence test of src/ops_lin_sol.c:383-394, on squares, and beta for
+        // the next step
+        int leave = -1;
+        total(0, [&](int c, double rr) {
+            if (c >= k || !s_act[c]) return;
+            const double be = scalar_quotient<T>(rr, sc->rho1[c]);
+            sc->rho2[c] = rr;
+            sc->beta[c] = be;
+            s_coef[c] = (T)be;
+            if (!(rr > stop[c])) {
+                sc->active[c] = 0;
+                sc->left_at[c] = it + 1;
+                leave = c;
+            }
+        });
+        const int left = __syncthreads_count(leave >= 0);
+        if (leave >= 0) s_act[leave] = 0;
+        if (tid == 0) {
+            s_nactive -= left;
+            sc->nactive = s_nactive;
+            sc->niter = it + 1;
+        }
+        __syncthreads();
     }
     finish(true);
 }
 
 // ---------------------------------------------------------------- small operators
-// Grid-wide barrier number `epoch` without a last block's turn: every block
-// waits for the arrivals of all.  Bounded as grid_sync is.
-__device__ __forceinline__ bool grid_arrive_wait(PcgSync *gs, int *error,
-                                                 unsigned long long timeout_ns,
-                                                 long long max_polls, unsigned long long epoch) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_ok = 1;
-        __threadfence();
-        const unsigned long long all = epoch * gridDim.x;
-        if (atomicAdd(&gs->arrive, 1ull) + 1ull < all) {
-            const unsigned long long t0 = global_ns();
-            for (long long poll = 0; ld_acquire(&gs->arrive) < all; ++poll) {
-                if ((poll & 31) == 31 &&
-                    (*(volatile int *)error != 0 || poll > max_polls ||
-                     global_ns() - t0 > timeout_ns)) {
-                    atomicExch(error, 1);
-                    s_ok = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 // The same block CG for operators whose step is a chain of latencies rather
 // than bytes or FMAs: phases of a microsecond between barriers.
 //
@@ -901,21 +903,6 @@ __device__ __forceinline__ void unit_gather(const int *col, const T *val, int wi
         unit_entries<T, GU, NE, RP>(col + 32 * e, val + 32 * e, width - e, V, Vp, beta, u0, G, acc);
 }
 
-// a / b for a coefficient that is used in T.  For FP32 the reciprocal's FP32 value
-// and one Newton step in FP64, y + y (1 - b y): three dependent FP64 operations
-// instead of a division's chain, and a relative error below 2^-45.
-template <typename T>
-__device__ __forceinline__ double scalar_quotient(double a, double b) {
-    if constexpr (sizeof(T) == 4) {
-        const double m = fabs(b);
-        if (m > 1e-30 && m < 1e30) {
-            const double y = (double)(1.0f / (float)b);
-            return a * fma(y, fma(-b, y, 1.0), y);
-        }
-    }
-    return a / b;
-}
-
 template <typename T, int GU, int U, bool CL, bool FUSE>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
@@ -942,7 +929,9 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k = a.k, n = a.n, G = kp / L, nch = (G + GU - 1) / GU;
     const int nb = gridDim.x, me = blockIdx.x;
-    const bool stats_block = me == 0;
+    const bool stats_thread = me == 0 && tid == kSmallThreads - 1;
+    __shared__ PcgTally<T> tally;
+    if (stats_thread) tally.clear();
     if (!CL && a.withhold_last && nb > 1 && me == nb - 1) return;
     if constexpr (CL) cooperative_groups::this_cluster().sync();  // all blocks run
 
@@ -1031,68 +1020,33 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
     auto part_of = [&](unsigned long long e, int which) {
         return a.part + ((size_t)(e & 1) * 2 + which) * nb * kp;
     };
-    // Column sums over `count` values get(b, c): Q lanes of a warp a column, each
-    // every Q-th value, then a tree over the lanes; use(c, sum, q) on all of
-    // them.  (An FP64 addition occupies a scheduler for 64 clocks whatever the
-    // lanes at work: a column's chain is kept short and few warps take part.)
-    const int Q = kp <= 16 ? 8 : 4;
-    auto col_sums = [&](int count, auto get, auto use) {
-        if (tid >= ((kp * Q + 31) & ~31)) return;
-        const int c = tid / Q, q = tid % Q;
-        double t = 0.0;
-        if (c < kp && q < count) {
-            t = get(q, c);
-            for (int b = q + Q; b < count; b += Q) t += get(b, c);
-        }
-        for (int o = Q / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (c < kp) use(c, t, q);
-    };
     // this block's column sums of wred, for the next barrier: into the other
     // blocks' shared memory in a cluster, else into global memory
     auto publish = [&](int which) {
         __syncthreads();
-        col_sums(
-            nsl, [&](int sl, int c) { return (double)wred[sl * nch + c / CC][c % CC]; },
+        lane_cols_sum(
+            kp, nsl, [&](int sl, int c) { return (double)wred[sl * nch + c / CC][c % CC]; },
             [&](int c, double t, int q) {
                 if constexpr (CL) {
                     double *at = stripe + ((((epoch + 1) & 1) * 2 + which) * nb + me) * kp + c;
-                    for (int b = q; b < nb; b += Q)
+                    for (int b = q; b < nb; b += kp <= 16 ? 8 : 4)
                         *cooperative_groups::this_cluster().map_shared_rank(at, b) = t;
                 } else if (q == 0) {
                     part_of(epoch + 1, which)[(size_t)me * kp + c] = t;
                 }
             });
     };
-    // Sums of the partials over the blocks, used by lane 0 of each column's;
-    // the caller synchronises the block.  From global memory `stripes` threads a
-    // column first add a fixed share of the blocks each.
+    // sums of the partials over the blocks; the caller synchronises the block
     auto total = [&](int which, auto use) {
-        auto first = [&](int c, double t, int q) {
-            if (q == 0) use(c, t);
-        };
         if constexpr (CL) {
             const double *part = stripe + ((epoch & 1) * 2 + which) * nb * kp;
-            col_sums(nb, [&](int b, int c) { return part[b * kp + c]; }, first);
+            lane_cols_sum(
+                kp, nb, [&](int b, int c) { return part[b * kp + c]; },
+                [&](int c, double t, int q) {
+                    if (q == 0) use(c, t);
+                });
         } else {
-            const double *part = part_of(epoch, which);
-            const int stripes = min(min(kSmallThreads / kp, 32), nb);
-            const int c = tid % kp, st = tid / kp;
-            if (st < stripes) {
-                double t0 = __ldcg(part + (size_t)st * kp + c);
-                double t1 = 0.0;
-                int b = st + stripes;
-                if (b < nb) t1 = __ldcg(part + (size_t)b * kp + c);
-                for (b += stripes; b + stripes < nb; b += 2 * stripes) {
-                    const double v0 = __ldcg(part + (size_t)b * kp + c);
-                    const double v1 = __ldcg(part + (size_t)(b + stripes) * kp + c);
-                    t0 += v0;
-                    t1 += v1;
-                }
-                if (b < nb) t0 += __ldcg(part + (size_t)b * kp + c);
-                stripe[tid] = t0 + t1;
-            }
-            __syncthreads();
-            col_sums(stripes, [&](int st, int c) { return stripe[st * kp + c]; }, first);
+            grid_cols_sum<kSmallThreads>(part_of(epoch, which), nb, kp, stripe, use);
         }
     };
     auto barrier = [&]() {
@@ -1122,6 +1076,7 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             a.stats->launches += 1;
             a.stats->iters += (unsigned long long)sc->niter;
         }
+        if (stats_thread) tally.write(a, kp);
     };
 
     // ---------------- r = b - S x (or r = b for x = 0), p = 0, norms
@@ -1200,8 +1155,6 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
         for (int c = 0; c < k; ++c) cnt += s_act[c];
         s_nactive = sc->nactive = cnt;
         sc->niter = 0;
-        if (stats_block)
-            a.stats->kernel_bytes += (a.x_zero ? 0.0 : a.matrix_bytes) + 4.0 * n * kp * sizeof(T);
     }
     __syncthreads();
 
@@ -1230,7 +1183,7 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
                 return;
             }
         }
-        if (tid == 0 && stats_block) gs->t_spmm = global_ns();
+        if (stats_thread) tally.begin();
         // ---------------- w = S p, p^T w
 #pragma unroll
         for (int i = 0; i < U; ++i) {
@@ -1261,17 +1214,14 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             sc->alpha[c] = al;
             s_alpha[c] = (T)al;
         });
-        if (tid == kSmallThreads - 1 && stats_block) {
+        if (stats_thread) {
             int gact = 0;
             for (int u = 0; u < G; ++u) {
                 int any = 0;
                 for (int l = 0; l < L; ++l) any |= s_act[u * L + l];
                 gact += any != 0;
             }
-            const double vec = (double)n * gact * L * sizeof(T);
-            a.stats->spmm_ns += global_ns() - gs->t_spmm;
-            a.stats->spmm_bytes += a.matrix_bytes + 2.0 * vec;
-            a.stats->kernel_bytes += a.matrix_bytes + 12.0 * vec;
+            tally.end(gact);
         }
         __syncthreads();
         // ---------------- x += alpha p, r -= alpha w, r^T r
@@ -1466,20 +1416,17 @@ bool launch_pcg_small(const PcgArgs<T> &a, int kp, cudaStream_t st) {
     return true;
 }
 
-constexpr int kMaxBlocksPerSm = 4;
-
 template <typename T, int KP>
 void launch_block_pcg(PcgArgs<T> a, cudaStream_t st) {
-    static PerDevice<int> occupancy;
-    const int bpsm = occupancy.get([] {
+    static PerDevice<bool> fits;
+    GCGE_REQUIRE(fits.get([] {
         int b = 0;
         GCGE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_block_pcg<T, KP>,
                                                                 pcg_threads<T, KP>(), 0));
-        return std::min(b, kMaxBlocksPerSm);
-    });
-    GCGE_REQUIRE(bpsm >= 1, GCGE_ERR_CUDA, "block PCG: kernel does not fit on an SM");
-    const int nb =
-        std::max(1, std::min(bpsm * device_sms() / std::max(1, t_pcg_share), a.nslices));
+        return b >= 1;
+    }),
+                 GCGE_ERR_CUDA, "block PCG: kernel does not fit on an SM");
+    const int nb = std::max(1, std::min(device_sms() / std::max(1, t_pcg_share), a.nslices));
     void *args[] = {&a};
     GCGE_CUDA(cudaLaunchCooperativeKernel((const void *)k_block_pcg<T, KP>, dim3(nb),
                                           dim3(pcg_threads<T, KP>()), args, 0, st));
