@@ -775,27 +775,37 @@ void fill_value(size_t count, double *X, double v, cudaStream_t st) {
 
 namespace gcge {
 
+// max |C_ij| into *out, which may be page-locked host memory (the callers wait
+// for the stream before they read it: no copy of its own).  On the bits, which
+// order as the magnitudes do, a NaN above all: an FP64 comparison occupies a
+// scheduler for 64 clocks, and a block of them made this 9 us for 240 entries.
 __global__ void k_absmax(int m, int w, const double *__restrict__ C, int ldc, double *out) {
-    __shared__ double red[32];
-    double v = 0.0;
+    __shared__ unsigned long long red[32];
+    unsigned long long v = 0;
     for (int e = threadIdx.x; e < m * w; e += blockDim.x) {
-        const double a = fabs(C[(e % m) + (size_t)(e / m) * ldc]);
-        v = (a > v || a != a) ? a : v;
+        const unsigned long long a =
+            (unsigned long long)__double_as_longlong(C[(e % m) + (size_t)(e / m) * ldc]) << 1;
+        v = a > v ? a : v;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        const double u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = (u > v || u != u) ? u : v;
-    }
+    auto warp_max = [](unsigned long long x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long u = __shfl_xor_sync(0xffffffffu, x, o);
+            x = u > x ? u : x;
+        }
+        return x;
+    };
+    v = warp_max(v);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0.0;
-        for (int i = 0; i < (int)(blockDim.x + 31) / 32; ++i) r = (red[i] > r || red[i] != red[i]) ? red[i] : r;
-        *out = r;
+    if (threadIdx.x < 32) {
+        v = warp_max(threadIdx.x < (blockDim.x + 31) / 32 ? red[threadIdx.x] : 0ull);
+        if (threadIdx.x == 0) *out = __longlong_as_double((long long)(v >> 1));
     }
 }
 void absmax(int m, int w, const double *C, int ldc, double *out, cudaStream_t st) {
-    k_absmax<<<1, 1024, 0, st>>>(m, w, C, ldc, out);
+    const int threads = (int)std::min<long long>(1024, ((long long)m * w + 31) / 32 * 32);
+    k_absmax<<<1, std::max(threads, 32), 0, st>>>(m, w, C, ldc, out);
     GCGE_CHECK_LAUNCH();
     count_launch();
 }

@@ -96,7 +96,6 @@ void SolverCtx::reserve(int n_, int nev_max, int nev_init, int bs, int spmm_nblo
                                 2u << 20));
     part.alloc((size_t)std::max(spmm_nblocks, 1) * 64);
     ozb.alloc(oz_lincomb_scratch_bytes(std::max(smax, cols), std::max(smax, cols)));
-    dmax.alloc(4);
     hmax.alloc(4);
     if (one.p == nullptr) {
         one.alloc(1);
@@ -216,8 +215,7 @@ int borth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int start, 
         }
     };
     auto device_absmax = [&](int m, int w, const double *C, int ldc) {
-        absmax(m, w, C, ldc, c.dmax.p, st);
-        GCGE_CUDA(cudaMemcpyAsync(c.hmax.p, c.dmax.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+        absmax(m, w, C, ldc, c.hmax.p, st);
         GCGE_CUDA(cudaStreamSynchronize(st));
         return c.hmax.p[0];
     };
@@ -375,8 +373,7 @@ struct BgsOrth {
         }
     }
     double absmax_dev(int m, int w, const double *C, int ldc) {
-        absmax(m, w, C, ldc, c.dmax.p, st);
-        GCGE_CUDA(cudaMemcpyAsync(c.hmax.p, c.dmax.p, sizeof(double), cudaMemcpyDeviceToHost, st));
+        absmax(m, w, C, ldc, c.hmax.p, st);
         GCGE_CUDA(cudaStreamSynchronize(st));
         return c.hmax.p[0];
     }
@@ -595,13 +592,6 @@ struct GcgRun {
             copy_cols(n, k, X, ldx, Y, ldy, st);
         }
     }
-    double device_absmax(int m, int w, const double *C, int ldc) {
-        absmax(m, w, C, ldc, c.dmax.p, st);
-        GCGE_CUDA(cudaMemcpyAsync(c.hmax.p, c.dmax.p, sizeof(double), cudaMemcpyDeviceToHost, st));
-        GCGE_CUDA(cudaStreamSynchronize(st));
-        return c.hmax.p[0];
-    }
-
     // MultiVecOrth with the method the parameters select ("bgs": binary
     // Gram-Schmidt; anything else: the GPU counterpart of modified
     // Gram-Schmidt, src/ops_eig_sol_gcg.c:119-141, :396-419, :650-668)
