@@ -10,58 +10,71 @@ namespace gcge {
 // blocked block sits at ((i / 32) G + c / L) 32 L + (i % 32) L + c % L with
 // L = 16 / sizeof(T), G = kp / L; rows up to the next multiple of 32 and
 // columns k..kp-1 are zero.
-template <typename T>
-__host__ __device__ __forceinline__ size_t blk_index(int i, int c, int kp) {
-    constexpr int L = 16 / (int)sizeof(T);
-    const int G = kp / L;
-    return ((size_t)(i >> 5) * G + c / L) * (32 * L) + (size_t)(i & 31) * L + c % L;
-}
+//
+// A warp converts one 16-byte column group of one slice, a row per lane: whole
+// 256-byte runs of every column on one side, one 512-byte run on the other, and
+// one division per 32 rows instead of two or three 64-bit ones per element
+// (128^3 rows x 40 columns, FP64 to FP32 and back, 1.0 GB each: 252 and 259 us with
+// those, 156 and 159 now).
 template <typename S, typename T>
-__global__ void k_col_to_rows(int n, int k, int kp, const S *__restrict__ X, int ldx,
-                              T *__restrict__ Y) {
+__global__ void __launch_bounds__(256)
+k_col_to_rows(int n, int k, int kp, const S *__restrict__ X, int ldx, T *__restrict__ Y) {
     constexpr int L = 16 / (int)sizeof(T);
-    const int G = kp / L;
-    const size_t total = (size_t)((n + 31) / 32) * 32 * kp;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-         t += (size_t)gridDim.x * blockDim.x) {
-        // t = ((s G + u) 32 + l) L + e
-        const int e = (int)(t % L);
-        const size_t q = t / L;
-        const int l = (int)(q % 32);
-        const size_t su = q / 32;
-        const int u = (int)(su % G);
-        const int i = (int)(su / G) * 32 + l, c = u * L + e;
-        Y[t] = (i < n && c < k) ? (T)X[i + (size_t)c * ldx] : T(0);
+    const int G = kp / L, lane = threadIdx.x & 31;
+    const long long units = (long long)((n + 31) / 32) * G;
+    for (long long w = blockIdx.x * 8ll + (threadIdx.x >> 5); w < units; w += gridDim.x * 8ll) {
+        const int s = (int)(w / G), u = (int)(w - (long long)s * G), i = s * 32 + lane;
+        struct alignas(16) {
+            T v[L];
+        } o;
+#pragma unroll
+        for (int e = 0; e < L; ++e) {
+            const int c = u * L + e;
+            o.v[e] = (i < n && c < k) ? (T)X[i + (size_t)c * ldx] : T(0);
+        }
+        *reinterpret_cast<decltype(o) *>(Y + (size_t)w * 32 * L + lane * L) = o;
     }
 }
 // add: Y += X where X is finite.  On an indefinite operator a column of the FP32
 // correction can leave the range of its type (a nearly vanishing p^T S p); such
 // a column of Y stays as it was instead of spoiling the block it belongs to.
 template <typename T, typename D>
-__global__ void k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y,
-                              int ldy, int add) {
-    const size_t total = (size_t)n * k;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-         t += (size_t)gridDim.x * blockDim.x) {
-        const int c = (int)(t / n), i = (int)(t % n);
-        const D v = (D)X[blk_index<T>(i, c, kp)];
-        D &y = Y[i + (size_t)c * ldy];
-        y = add ? (isfinite(v) ? y + v : y) : v;
+__global__ void __launch_bounds__(256)
+k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, int ldy, int add) {
+    constexpr int L = 16 / (int)sizeof(T);
+    const int G = kp / L, used = (k + L - 1) / L, lane = threadIdx.x & 31;
+    const long long units = (long long)((n + 31) / 32) * used;
+    for (long long w = blockIdx.x * 8ll + (threadIdx.x >> 5); w < units; w += gridDim.x * 8ll) {
+        const int s = (int)(w / used), u = (int)(w - (long long)s * used), i = s * 32 + lane;
+        struct alignas(16) Pack {
+            T v[L];
+        };
+        const Pack q = *reinterpret_cast<const Pack *>(X + ((size_t)s * G + u) * 32 * L + lane * L);
+        if (i >= n) continue;
+#pragma unroll
+        for (int e = 0; e < L; ++e) {
+            const int c = u * L + e;
+            if (c >= k) continue;
+            const D v = (D)q.v[e];
+            D &y = Y[i + (size_t)c * ldy];
+            y = add ? (isfinite(q.v[e]) ? y + v : y) : v;
+        }
     }
 }
 
 template <typename S, typename T>
 void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t st) {
-    const size_t total = (size_t)((n + 31) / 32) * 32 * kp;
-    const int g = (int)std::max<size_t>(1, std::min<size_t>((total + 255) / 256, 16 * device_sms()));
+    const long long units = (long long)((n + 31) / 32) * (kp / (16 / (int)sizeof(T)));
+    const int g = (int)std::max(1ll, std::min((units + 7) / 8, 16ll * device_sms()));
     k_col_to_rows<S, T><<<g, 256, 0, st>>>(n, k, kp, X, ldx, Y);
     GCGE_CHECK_LAUNCH();
     count_launch();
 }
 template <typename T, typename D>
 void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st) {
-    const size_t total = (size_t)n * k;
-    const int g = (int)std::max<size_t>(1, std::min<size_t>((total + 255) / 256, 16 * device_sms()));
+    constexpr int L = 16 / (int)sizeof(T);
+    const long long units = (long long)((n + 31) / 32) * ((k + L - 1) / L);
+    const int g = (int)std::max(1ll, std::min((units + 7) / 8, 16ll * device_sms()));
     k_rows_to_col<T, D><<<g, 256, 0, st>>>(n, k, kp, X, Y, ldy, add ? 1 : 0);
     GCGE_CHECK_LAUNCH();
     count_launch();
