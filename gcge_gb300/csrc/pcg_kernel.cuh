@@ -658,6 +658,16 @@ k_block_pcg(PcgArgs<T> a) {
             bool ga[G];
 #pragma unroll
             for (int u = 0; u < G; ++u) ga[u] = s_gact[u] != 0;
+            // FP32, while every group is active: two entries' loads in flight per
+            // lane instead of one's (30 steps, 64^3 27-point: k = 8 1498 -> 1178 us,
+            // k = 28 4070 -> 3444; 72^3 7-point: 825 -> 789, 3629 -> 3415).  Not at 16
+            // and 20 columns, whose 64 registers are few for the loads (72^3, k = 20
+            // 2116 -> 2135; 64^3 27-point 2568 -> 2401), nor in FP64, which its FMAs
+            // bound.
+            constexpr bool two_entries = sizeof(T) == 4 && (KP < 16 || KP > 20);
+            bool all_active = true;
+#pragma unroll
+            for (int u = 0; u < G; ++u) all_active &= ga[u];
             for (int s = s0 + warp; s < s1; s += nwarps) {
                 const long long beg = a.sp[s], end = a.sp[s + 1];
                 const int width = (int)((end - beg) >> 5);
@@ -696,7 +706,10 @@ k_block_pcg(PcgArgs<T> a) {
                     T acc[KP];
 #pragma unroll
                     for (int c = 0; c < KP; ++c) acc[c] = T(0);
-                    gather_row<T, KP>(a.col, a.val, beg + lane, width, a.P, ga, acc);
+                    if (two_entries && all_active)
+                        gather_row_part<T, KP, 0, G>(a.col, a.val, beg + lane, width, a.P, acc);
+                    else
+                        gather_row<T, KP>(a.col, a.val, beg + lane, width, a.P, ga, acc);
                     const int row = s * 32 + lane;
                     if (row < n) {
 #pragma unroll
