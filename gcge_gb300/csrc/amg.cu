@@ -9,7 +9,7 @@
 // The V-cycle runs on the host through the OPS slots, as in the reference:
 // at level l, BlockPCG smoothing with that level's iteration cap, rate and
 // tolerance (installed by MultiLinearSolverSetup_BlockPCG, so the smoothing
-// is the persistent block-PCG kernel of pcg.cu on the level's matrix), the
+// is the persistent block-PCG kernel of pcg_kernel.cuh on the level's matrix), the
 // residual b - A_l x, its restriction P_l^T r, the coarse solve from zero,
 // the prolongation P_l e added to x, and the post-smoothing; the coarsest
 // level is one BlockPCG solve.  Cycles repeat until the residual field of the

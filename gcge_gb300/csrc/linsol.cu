@@ -8,7 +8,7 @@
 // layout, whose niter / residual the solve fills in.  The solve takes one of
 // two routes with the same iteration:
 //  * no operator callback (MatDotMultiVec NULL), a CUDA matrix, and an "abs"
-//    or "rel" tolerance: the persistent block-PCG kernel (pcg.cu), one launch
+//    or "rel" tolerance: the persistent block-PCG kernel (pcg_kernel.cuh), one launch
 //    per 40 columns (the columns are independent CG solves);
 //  * otherwise (the caller's operator callback, e.g. the reference's shifted
 //    product MatDotMultiVecShift, or the "user" tolerance with norms from

@@ -1,6 +1,6 @@
 // Sparse kernels on SELL-32 matrices: SpMM over a block of columns and the
 // fused residual norm ||(A - lambda_c B) x_c||^2 of CheckConvergence (the
-// block-PCG SpMM lives inside the persistent kernel of pcg.cu).
+// block-PCG SpMM lives inside the persistent kernels of pcg_kernel.cuh).
 //
 // Layout: one warp owns one 32-row slice; lane l owns row 32*slice + l and
 // walks the slice's entries e = 0..width-1 at slice_ptr + e*32 + l, so each

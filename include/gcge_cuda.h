@@ -264,8 +264,9 @@ int GCGE_BlockPCG(void *A, void *B, double sigma, void **b, void **x, int k, int
  * timeout_ms and the grid's last block leaving before its first barrier, so
  * the other blocks' waits run out.  Expected result: GCGE_ERR_CUDA, with the
  * device context intact (the next solve succeeds).  Needs an operator large
- * enough for the grid form (FP64: more slices than a 16-CTA cluster has
- * warps, n > 4096 or so).  No counterpart in the reference. */
+ * enough for a grid barrier (the smallest run as one cluster, which waits in
+ * hardware: FP64 5-point operators up to n k of 12800 or so).  No counterpart
+ * in the reference. */
 int GCGE_TestBlockPCGBarrierTimeout(void *A, void **b, void **x, int k, double timeout_ms);
 /* B-orthonormalise columns [start, *end) of x against [0, start) (B NULL =
  * identity), as MultiVecOrth does (src/ops_orth.c:203-394); *end shrinks by
