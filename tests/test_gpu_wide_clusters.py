@@ -35,3 +35,12 @@ def test_cluster_wider_than_the_block(gpu_lib, seed, mixed):
     V = r.evec[:, :22]
     res = np.linalg.norm(P.laplace3d(44).to_scipy() @ V - V * r.eval[:22], axis=0)
     assert np.all(res <= 7.5e-10 * r.eval[:22])
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_stall_far_from_the_tolerance_goes_over_to_fp64(gpu_lib, seed):
+    """From some starting blocks the mixed solve stalls at a few hundred times
+    its tolerance; FP64 takes about 95 iterations, so twice as many are a stall
+    that was not noticed."""
+    r = cube_solve(gpu_lib, seed, True)
+    assert r.status == gpu_lib.GCGE_OK and r.niter < 190
