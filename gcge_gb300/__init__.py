@@ -45,7 +45,7 @@ EXPORTED_SYMBOLS = [
     "GCGE_ServerSubmit", "GCGE_ServerWait", "GCGE_ServerDestroy", "GCGE_SolveBatch",
     "MultiVecOrthSetup_ModifiedGramSchmidt", "MultiVecOrthSetup_BinaryGramSchmidt",
     "EigenSolverSetParametersFromCommandLine_GCG", "CUDA_MatAxpby",
-    "MultiLinearSolverSetup_BlockPCG", "GCGE_TestBlockPCGBarrierTimeout",
+    "MultiLinearSolverSetup_BlockPCG", "GCGE_TestBlockPCGBarrierTimeout", "GCGE_MixedInnerSolve",
     "GCGE_BenchDenseProduct", "GCGE_SetSpMMTuning", "GCGE_SpMMTuneCandidates", "GCGE_SpMMTune",
     "CUDA_TransferCreateFromCCS", "CUDA_TransferDestroy", "CUDA_MultiVecFromItoJ",
     "MultiLinearSolverSetup_BlockAMG",

@@ -20,6 +20,7 @@
 #include <array>
 #include <chrono>
 #include <cmath>
+#include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
@@ -554,6 +555,19 @@ int bgs_orth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int star
 }
 
 // ---------------------------------------------------------------- the solve
+// The FP32 part of a mixed inner solve: CG from 0 on S d = r (r in c.r64, S's FP32
+// values formed), x += d accumulated in FP64, but for the columns of d that left
+// FP32's range (c.pcg.h_out, once the stream has passed).
+void mixed_correction(SolverCtx &c, int n, int k, double *x, int ldx, int max_iter, double rate,
+                      double tol, bool rel, cudaStream_t st) {
+    const int kp = rows_width(k, 4);
+    col_to_rows<double, float>(n, k, kp, c.r64.p, c.ld, c.br32.p, st);
+    block_pcg_rows<float>(c.pcg, c.upat, c.us32.p, c.br32.p, c.xr32.p, c.rr32.p, c.pr32.p,
+                          c.wr32.p, kp, k, max_iter, rate, tol, rel, true, st);
+    rows_to_col<float, double>(n, k, kp, c.xr32.p, x, ldx, true, st, &c.pcg.sync.p->out_of_range,
+                               c.pcg.h_out.p);
+}
+
 struct GcgRun {
     SolverCtx &c;
     GCGSolver &g;
@@ -789,12 +803,9 @@ struct GcgRun {
                    cur.first <= old.first && cur.second > 0.5 * old.second;
         };
         if (stalled(10, 100.0) || (first_rel <= 1e-3 && stalled(30, 1e4))) {
-            c.escalated = true;
-            escalated_at = iter_print + 1;
-            restart_pending = true;
-            if (g.print)
-                printf("%3d mixed precision: residual %6.5e stalled near the tolerance, FP64 from here\n",
-                       escalated_at, first_rel);
+            char why[64];
+            std::snprintf(why, sizeof why, "residual %6.5e stalled near the tolerance", first_rel);
+            escalate(why);
         }
     }
 
@@ -934,6 +945,7 @@ struct GcgRun {
         endW = orth(colp(V, 0), ld, n, startW, endW, B != nullptr, g.compW_orth_zero_tol,
                     g.compW_orth_max_reorth, g.compW_orth_method, g.compW_orth_block_size);
         sizeW = endW - startW;
+        if (mixed && ud != 1 && bsz > 0) check_corrections(bsz);
     }
 
     // BlockPCG on S x = b (b in c.bbuf, S = A + sigma B on the union pattern,
@@ -954,20 +966,40 @@ struct GcgRun {
         } else {
             // CG from x0 on S x = b is CG from 0 on S d = b - S x0: the residual
             // is formed in FP64 (it is a difference of nearly equal vectors once
-            // the Ritz vectors converge), the correction d is iterated in FP32,
-            // and x = x0 + d is accumulated in FP64.
-            const int kp = rows_width(bsz, 4);
+            // the Ritz vectors converge)
             if (!have_sx) {  // else r64 already holds S x
                 spmm<double>(c.upat, c.us64.p, x, ld, c.r64.p, ld, bsz, st);
                 spmm_calls++;
             }
             axpby(n, bsz, 1.0, c.bbuf.p, ld, -1.0, c.r64.p, ld, st);
-            col_to_rows<double, float>(n, bsz, kp, c.r64.p, ld, c.br32.p, st);
-            block_pcg_rows<float>(c.pcg, c.upat, c.us32.p, c.br32.p, c.xr32.p, c.rr32.p,
-                                  c.pr32.p, c.wr32.p, kp, bsz, g.compW_cg_max_iter,
-                                  g.compW_cg_rate, g.compW_cg_tol, rel, true, st);
-            rows_to_col<float, double>(n, bsz, kp, c.xr32.p, x, ld, true, st);
+            mixed_correction(c, n, bsz, x, ld, g.compW_cg_max_iter, g.compW_cg_rate,
+                             g.compW_cg_tol, rel, st);
         }
+    }
+
+    // After the orthogonalisation of W (which waited for the stream): the columns
+    // whose FP32 correction left the range of its type kept their Ritz vector
+    // and were dropped as dependent.  A few may be, for a while: the shift of an
+    // early iteration is indefinite.  When the operator puts every column out of
+    // range the mixed solve has no direction to go on with, and when some stay
+    // out (a shift that hits an eigenvalue) the rest of it runs in FP64.
+    static constexpr int kOutIters = 3;
+    int out_iters = 0;
+    void check_corrections(int bsz) {
+        const unsigned long long out = *c.pcg.h_out.p;
+        if (out == 0) {
+            out_iters = 0;
+            return;
+        }
+        GCGE_REQUIRE(__builtin_popcountll(out) < bsz, GCGE_ERR_NUMERIC,
+                     "ComputeW: every FP32 correction left the range of its type");
+        if (++out_iters >= kOutIters) escalate("FP32 corrections out of range");
+    }
+    void escalate(const char *why) {
+        c.escalated = true;
+        escalated_at = iter_print + 1;
+        restart_pending = true;
+        if (g.print) printf("%3d mixed precision: %s, FP64 from here\n", escalated_at, why);
     }
 
     // The A x and B x of Ritz-vector columns [o1, o2) are in c.chkA / c.chkB.
@@ -1027,6 +1059,7 @@ struct GcgRun {
         endW = orth(colp(V, 0), ld, n, startW, endW, B != nullptr, g.compW_orth_zero_tol,
                     g.compW_orth_max_reorth, g.compW_orth_method, g.compW_orth_block_size);
         sizeW = endW - startW;
+        if (mixed && bsz > 0) check_corrections(bsz);
     }
 
     // ---------------- ComputeRayleighRitz (:931-1258)

@@ -74,6 +74,9 @@ int borth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int start, 
 // borth plus the leaf size (<= 0: the reference's default choice).
 int bgs_orth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int start, int end,
              bool useB, double zero_tol, int max_reorth, int block_size, int *spmm_calls);
+// The FP32 part of a mixed solve's inner solve (x += d, S d = r64 by block CG).
+void mixed_correction(SolverCtx &c, int n, int k, double *x, int ldx, int max_iter, double rate,
+                      double tol, bool rel, cudaStream_t st);
 // Union pattern of A, B (B NULL = identity) and the diagonal, with A's and B's
 // values on it; cached on the context by matrix identity.
 void prepare_union(SolverCtx &c, SparseMat *A, SparseMat *B, cudaStream_t st);

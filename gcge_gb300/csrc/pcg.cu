@@ -35,13 +35,36 @@ k_col_to_rows(int n, int k, int kp, const S *__restrict__ X, int ldx, T *__restr
         *reinterpret_cast<decltype(o) *>(Y + (size_t)w * 32 * L + lane * L) = o;
     }
 }
-// add: Y += X where X is finite.  On an indefinite operator a column of the FP32
-// correction can leave the range of its type (a nearly vanishing p^T S p); such
-// a column of Y stays as it was instead of spoiling the block it belongs to.
+// *out |= a bit for each column of X (slice-blocked, FP32) with an entry that is
+// not finite.  X once at HBM speed; a kernel of its own, as the solve's kernels
+// have no register left for it (k_block_pcg<float, 20> spilled 36 bytes
+// instead of 20).
+__global__ void __launch_bounds__(256)
+k_out_of_range(int n, int kp, const float *__restrict__ X, unsigned long long *out) {
+    const int G = kp / 4, lane = threadIdx.x & 31;
+    const long long units = (long long)((n + 31) / 32) * G;
+    unsigned long long bits = 0;
+    for (long long w = blockIdx.x * 8ll + (threadIdx.x >> 5); w < units; w += gridDim.x * 8ll) {
+        const int s = (int)(w / G), u = (int)(w - (long long)s * G);
+        const float4 v = *reinterpret_cast<const float4 *>(X + (size_t)w * 128 + lane * 4);
+        if (s * 32 + lane >= n) continue;
+        const unsigned bad = (isfinite(v.x) ? 0u : 1u) | (isfinite(v.y) ? 0u : 2u) |
+                             (isfinite(v.z) ? 0u : 4u) | (isfinite(v.w) ? 0u : 8u);
+        bits |= (unsigned long long)bad << (4 * u);
+    }
+    if (bits) atomicOr(out, bits);
+}
+// add: Y += X.  On an indefinite operator a column of the FP32 correction can
+// leave the range of its type (a nearly vanishing p^T S p); such a column of Y
+// (its bit in *skip) stays as it was, whole, instead of spoiling the block it
+// belongs to, and *report tells the host.
 template <typename T, typename D>
 __global__ void __launch_bounds__(256)
-k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, int ldy, int add) {
+k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, int ldy, int add,
+              const unsigned long long *skip, unsigned long long *report) {
     constexpr int L = 16 / (int)sizeof(T);
+    const unsigned long long out = skip ? *skip : 0ull;
+    if (report && blockIdx.x == 0 && threadIdx.x == 0) *report = out;
     const int G = kp / L, used = (k + L - 1) / L, lane = threadIdx.x & 31;
     const long long units = (long long)((n + 31) / 32) * used;
     for (long long w = blockIdx.x * 8ll + (threadIdx.x >> 5); w < units; w += gridDim.x * 8ll) {
@@ -54,10 +77,10 @@ k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, 
 #pragma unroll
         for (int e = 0; e < L; ++e) {
             const int c = u * L + e;
-            if (c >= k) continue;
+            if (c >= k || ((out >> c) & 1ull)) continue;
             const D v = (D)q.v[e];
             D &y = Y[i + (size_t)c * ldy];
-            y = add ? (isfinite(q.v[e]) ? y + v : y) : v;
+            y = add ? y + v : v;
         }
     }
 }
@@ -71,20 +94,28 @@ void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t s
     count_launch();
 }
 template <typename T, typename D>
-void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st) {
+void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st,
+                 unsigned long long *out, unsigned long long *report) {
     constexpr int L = 16 / (int)sizeof(T);
     const long long units = (long long)((n + 31) / 32) * ((k + L - 1) / L);
     const int g = (int)std::max(1ll, std::min((units + 7) / 8, 16ll * device_sms()));
-    k_rows_to_col<T, D><<<g, 256, 0, st>>>(n, k, kp, X, Y, ldy, add ? 1 : 0);
+    if constexpr (sizeof(T) == 4) {
+        if (out) {
+            k_out_of_range<<<g, 256, 0, st>>>(n, kp, X, out);
+            GCGE_CHECK_LAUNCH();
+            count_launch();
+        }
+    }
+    k_rows_to_col<T, D><<<g, 256, 0, st>>>(n, k, kp, X, Y, ldy, add ? 1 : 0, out, report);
     GCGE_CHECK_LAUNCH();
     count_launch();
 }
 template void col_to_rows<double, double>(int, int, int, const double *, int, double *, cudaStream_t);
 template void col_to_rows<double, float>(int, int, int, const double *, int, float *, cudaStream_t);
 template void rows_to_col<double, double>(int, int, int, const double *, double *, int, bool,
-                                          cudaStream_t);
+                                          cudaStream_t, unsigned long long *, unsigned long long *);
 template void rows_to_col<float, double>(int, int, int, const float *, double *, int, bool,
-                                         cudaStream_t);
+                                         cudaStream_t, unsigned long long *, unsigned long long *);
 
 void PcgWork::timing_reset(cudaStream_t st) {
     ev_used = 0;
@@ -128,6 +159,8 @@ void PcgWork::reserve(int n, int kmax_) {
         stats.alloc(1);
         h_sc.alloc(1);
         h_stats.alloc(1);
+        h_out.alloc(1);
+        *h_out.p = 0;
         GCGE_CUDA(cudaMemsetAsync(stats.p, 0, sizeof(PcgStats), lib_stream()));
     }
 }

@@ -26,6 +26,7 @@ struct PcgSync {
     unsigned long long arrive;  // block arrivals at barriers, over the launch
     int error;                  // a barrier wait ran out of time
     int pad;
+    unsigned long long out_of_range;  // columns rows_to_col found not finite, a bit each
 };
 struct PcgStats {
     double kernel_bytes;         // algorithmic bytes of the whole solves
@@ -45,6 +46,7 @@ struct PcgWork {
     DevBuf<PcgStats> stats;
     PinnedBuf<PcgScalars> h_sc;
     PinnedBuf<PcgStats> h_stats;
+    PinnedBuf<unsigned long long> h_out;  // columns rows_to_col left out, a bit each
     // whole-kernel timing (event pairs) and algorithmic bytes of the solves
     std::vector<cudaEvent_t> ev;
     size_t ev_used = 0;
@@ -89,7 +91,11 @@ inline size_t pcg_block_elems(int n, int kp) { return (size_t)((n + 31) / 32) * 
 // Column-major (ld) <-> slice-blocked (kp) block conversions (pcg.cu).
 template <typename S, typename T>
 void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t st);
+// add: Y += X.  With `out` (FP32; a zeroed word in device memory) the columns of X
+// that are not finite are left out, whole, and have a bit each in *out and in
+// *report (page-locked memory).
 template <typename T, typename D>
-void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st);
+void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st,
+                 unsigned long long *out = nullptr, unsigned long long *report = nullptr);
 
 }  // namespace gcge

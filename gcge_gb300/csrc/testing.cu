@@ -81,6 +81,37 @@ int GCGE_BlockPCG(void *A, void *B, double sigma, void **b, void **x, int k, int
     }
 }
 
+int GCGE_MixedInnerSolve(void *A, void *B, double sigma, void **b, void **x, int k, int max_iter,
+                         double rate, double tol, int *iters, unsigned long long *out_of_range) {
+    try {
+        SparseMat *Am = as_mat(A);
+        SparseMat *Bm = B ? as_mat(B) : nullptr;
+        MultiVec *bv = as_mv(b), *xv = as_mv(x);
+        GCGE_REQUIRE(Am && (!B || Bm) && bv && xv, GCGE_ERR_HANDLE, "GCGE_MixedInnerSolve: handles");
+        GCGE_REQUIRE(k >= 1 && k <= 40 && k <= bv->ncols && k <= xv->ncols, GCGE_ERR_ARG,
+                     "GCGE_MixedInnerSolve: k");
+        cudaStream_t st = lib_stream();
+        const int n = Am->n;
+        SolverCtx c;
+        prepare_union(c, Am, Bm, st);
+        c.reserve(n, k, k, k, spmm_blocks(c.upat));
+        const size_t nr = pcg_block_elems(n, rows_width(k, 4));
+        for (auto *v : {&c.xr32, &c.br32, &c.rr32, &c.pr32, &c.wr32}) v->alloc(nr);
+        shift_values(c.upat.padded, c.ua.p, c.ub.p, sigma, c.us64.p, c.us32.p, st);
+        spmm<double>(c.upat, c.us64.p, xv->data, xv->ld, c.r64.p, c.ld, k, st);
+        axpby(n, k, 1.0, bv->data, bv->ld, -1.0, c.r64.p, c.ld, st);
+        mixed_correction(c, n, k, xv->data, xv->ld, max_iter, rate, tol, false, st);
+        const int it = pcg_last_iters(c.pcg, st);
+        if (iters) *iters = it;
+        if (out_of_range) *out_of_range = *c.pcg.h_out.p;
+        return GCGE_OK;
+    } catch (const CudaError &e) {
+        set_error(e.status, e.where.c_str());
+        take_error();
+        return e.status;
+    }
+}
+
 int GCGE_TestBlockPCGBarrierTimeout(void *A, void **b, void **x, int k, double timeout_ms) {
     if (!(timeout_ms > 0.0)) return GCGE_ERR_ARG;
     struct Hook {

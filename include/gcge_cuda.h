@@ -39,7 +39,8 @@ enum {
     GCGE_ERR_ARG = 2,         /* invalid argument (size, range, NULL) */
     GCGE_ERR_ALLOC = 3,       /* device or host allocation failed */
     GCGE_ERR_HANDLE = 4,      /* handle is not a CUDA matrix / multivector */
-    GCGE_ERR_NUMERIC = 5,     /* NaN/Inf detected in residuals or projections */
+    GCGE_ERR_NUMERIC = 5,     /* NaN/Inf detected in residuals or projections, or (mixed
+                               * precision) an operator out of FP32's range */
     GCGE_ERR_NOT_CONVERGED = 6, /* numIterMax reached before nev pairs converged */
     GCGE_ERR_NO_DEVICE = 7,   /* no CUDA device visible */
     GCGE_ERR_TOO_LARGE = 8    /* projected problem exceeds the dense-solver capacity */
@@ -259,6 +260,12 @@ int GCGE_DenseEig(int s, const double *M, int ldm, double *eval, double *Z, int 
  * precision path. */
 int GCGE_BlockPCG(void *A, void *B, double sigma, void **b, void **x, int k, int max_iter,
                   double rate, double tol, int fp32, int *iters);
+/* The inner solve of a mixed-precision solve's W step: b - S x in FP64, block CG
+ * on the correction in FP32, x += correction in FP64 (absolute tolerance).
+ * *out_of_range: a bit for each column whose correction left the range of FP32;
+ * these columns of x are as they were. */
+int GCGE_MixedInnerSolve(void *A, void *B, double sigma, void **b, void **x, int k, int max_iter,
+                         double rate, double tol, int *iters, unsigned long long *out_of_range);
 /* Failure-detection test of the persistent block-PCG kernel's grid barrier:
  * GCGE_BlockPCG (FP64, sigma 0, 30 steps) with every barrier wait bounded by
  * timeout_ms and the grid's last block leaving before its first barrier, so
