@@ -663,8 +663,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
             }
         }
-        // all issued MMAs complete before tensor memory is freed
-        if (lane == 0) tc_commit(fin);
+        // all issued MMAs complete before tensor memory is freed.  A commit tracks
+        // the operations of its own thread: the lane that issued them (elect.sync
+        // picks the same lane for the same mask every time)
+        if (tc_elect()) tc_commit(fin);
         __syncwarp();
         mbar_wait_teardown(fin, 0);
     } else {
