@@ -540,6 +540,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     using L = TcLayout<BN, GRAM>;
     static_assert(BN % 16 == 0 && BN <= 64, "tile width: a multiple of 16, at most 64");
     constexpr int RH = L::halves, ACCS = L::accs;
+    // a linear combination's copies take two buffers from an even one on
+    static_assert(GRAM || RH == 4, "linear combination: raw buffers in pairs");
     extern __shared__ __align__(1024) uint8_t sm_raw[];
     // 1024-byte aligned base (the 128-byte swizzle of the bulk copies needs it)
     uint8_t *sm = sm_raw + ((1024u - (su32(sm_raw) & 1023u)) & 1023u);
