@@ -382,6 +382,15 @@ __device__ __forceinline__ double scalar_quotient(double a, double b) {
     return a / b;
 }
 
+// The r^T r at and below which a column leaves, !(|r| > u && |r| > v) on squares
+// (src/ops_lin_sol.c:383-394): negative bounds never stop a column, one that is
+// not a number does at once.
+__device__ __forceinline__ double stop_square(double u, double v) {
+    if (u != u || v != v) return u + v;
+    const double m = fmax(u, v);
+    return m < 0.0 ? -1.0 : m * m;
+}
+
 // Wide blocks (at least 8 column groups, an even number) gather the SpMM
 // phase in two halves of the column groups.
 template <typename T, int KP>
@@ -604,8 +613,7 @@ k_block_pcg(PcgArgs<T> a) {
             sc->last_res[c] = res;
             sc->alpha[c] = sc->beta[c] = 0.0;
             on = res > a.tol * nrm ? 1 : 0;
-            const double lim = fmax(a.rate * res, a.tol * nrm);
-            stop[c] = lim * lim;
+            stop[c] = stop_square(a.rate * res, a.tol * nrm);
         }
         sc->active[c] = on;
         sc->left_at[c] = 0;
@@ -1156,8 +1164,7 @@ k_pcg_small(PcgArgs<T> a, int kp, int smem_bytes) {
             sc->beta[c] = 0.0;
             sc->alpha[c] = 0.0;
             on = res > a.tol * nrm ? 1 : 0;
-            const double lim = fmax(a.rate * res, a.tol * nrm);
-            stop[c] = lim * lim;
+            stop[c] = stop_square(a.rate * res, a.tol * nrm);
         }
         sc->active[c] = s_act[c] = on;
         sc->left_at[c] = 0;
