@@ -367,16 +367,21 @@ __device__ __forceinline__ void grid_cols_sum(const double *part, int nb, int kp
         });
 }
 
-// a / b for a coefficient that is used in T.  For FP32 the reciprocal's FP32 value
-// and one Newton step in FP64, y + y (1 - b y): three dependent FP64 operations
-// instead of a division's chain, and a relative error below 2^-45.
+// a / b for a coefficient that is used in T.  For FP32 a quotient that rounds to the
+// same FP32 value: the divisor's reciprocal in FP32 and one Newton step in FP64,
+// y + y (1 - b y), whose relative error is at most (2^-23)^2 and a rounding, below
+// 130 units in the last place; three dependent FP64 operations instead of a
+// division's chain.  The division decides where that is too close to the middle of
+// two FP32 values (bits 28..0 at 2^28) or outside the normal FP32 range.
 template <typename T>
 __device__ __forceinline__ double scalar_quotient(double a, double b) {
     if constexpr (sizeof(T) == 4) {
         const double m = fabs(b);
         if (m > 1e-30 && m < 1e30) {
             const double y = (double)(1.0f / (float)b);
-            return a * fma(y, fma(-b, y, 1.0), y);
+            const double q = a * fma(y, fma(-b, y, 1.0), y), mag = fabs(q);
+            const int past = (__double2loint(q) & 0x1fffffff) - 0x10000000;
+            if (mag > 1.2e-38 && mag < 3.4e38 && abs(past) > 256) return q;
         }
     }
     return a / b;
