@@ -46,6 +46,7 @@ EXPORTED_SYMBOLS = [
     "MultiVecOrthSetup_ModifiedGramSchmidt", "MultiVecOrthSetup_BinaryGramSchmidt",
     "EigenSolverSetParametersFromCommandLine_GCG", "CUDA_MatAxpby",
     "MultiLinearSolverSetup_BlockPCG", "GCGE_TestBlockPCGBarrierTimeout", "GCGE_MixedInnerSolve",
+    "GCGE_TestBlockPCGForm", "GCGE_TestBlockPCGShare",
     "GCGE_BenchDenseProduct", "GCGE_SetSpMMTuning", "GCGE_SpMMTuneCandidates", "GCGE_SpMMTune",
     "CUDA_TransferCreateFromCCS", "CUDA_TransferDestroy", "CUDA_MultiVecFromItoJ",
     "MultiLinearSolverSetup_BlockAMG",

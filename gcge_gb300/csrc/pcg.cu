@@ -179,6 +179,7 @@ int pcg_last_iters(PcgWork &wk, cudaStream_t st) {
 }
 
 thread_local PcgBarrierTest t_pcg_barrier_test;
+thread_local PcgForm t_pcg_form = kPcgNone;
 
 template void block_pcg_rows<float>(PcgWork &, const SellPattern &, const float *, const float *,
                                     float *, float *, float *, float *, int, int, int, double,

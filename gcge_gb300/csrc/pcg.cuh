@@ -84,6 +84,9 @@ struct PcgBarrierTest {
     int withhold_last = 0;
 };
 extern thread_local PcgBarrierTest t_pcg_barrier_test;
+// Form of this thread's last block PCG launch, for the tests.
+enum PcgForm { kPcgNone = 0, kPcgCluster = 1, kPcgUnits = 2, kPcgPhases = 3 };
+extern thread_local PcgForm t_pcg_form;
 
 // Elements of a slice-blocked n x kp block (rows padded to a multiple of 32).
 inline size_t pcg_block_elems(int n, int kp) { return (size_t)((n + 31) / 32) * 32 * kp; }

@@ -1426,6 +1426,7 @@ bool launch_pcg_small(const PcgArgs<T> &a, int kp, cudaStream_t st) {
         work / csize <= cluster_clocks<T>(units(csize, 2) <= NW);
     const int nb = cluster ? csize : std::max(1, std::min(sms, a.nslices));
     if (!cluster && units(nb, 2) > 2 * NW) return false;
+    t_pcg_form = cluster ? kPcgCluster : kPcgUnits;
     // narrow chunks while every warp has one unit at most: more warps at work
     const int gu = units(nb, 1) <= NW ? 1 : 2, u = units(nb, gu) <= NW ? 1 : 2;
     auto go = [&](auto GU, auto U) {
@@ -1452,6 +1453,7 @@ void launch_block_pcg(PcgArgs<T> a, cudaStream_t st) {
     }),
                  GCGE_ERR_CUDA, "block PCG: kernel does not fit on an SM");
     const int nb = std::max(1, std::min(device_sms() / std::max(1, t_pcg_share), a.nslices));
+    t_pcg_form = kPcgPhases;
     void *args[] = {&a};
     GCGE_CUDA(cudaLaunchCooperativeKernel((const void *)k_block_pcg<T, KP>, dim3(nb),
                                           dim3(pcg_threads<T, KP>()), args, 0, st));

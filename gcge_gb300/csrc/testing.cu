@@ -126,6 +126,14 @@ int GCGE_TestBlockPCGBarrierTimeout(void *A, void **b, void **x, int k, double t
     return GCGE_BlockPCG(A, nullptr, 0.0, b, x, k, 30, 1e-2, 1e-14, 0, &it);
 }
 
+int GCGE_TestBlockPCGForm(void) { return (int)t_pcg_form; }
+
+int GCGE_TestBlockPCGShare(int workers) {
+    const int before = t_pcg_share;
+    t_pcg_share = workers;
+    return before;
+}
+
 int GCGE_BOrth(void *B, void **x, int start, int *end, double zero_tol, int max_reorth) {
     try {
         SparseMat *Bm = B ? as_mat(B) : nullptr;

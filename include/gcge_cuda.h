@@ -275,6 +275,13 @@ int GCGE_MixedInnerSolve(void *A, void *B, double sigma, void **b, void **x, int
  * hardware: FP64 5-point operators up to n k of 12800 or so).  No counterpart
  * in the reference. */
 int GCGE_TestBlockPCGBarrierTimeout(void *A, void **b, void **x, int k, double timeout_ms);
+/* Which form this thread's last block CG ran in: 1 one thread-block cluster, 2
+ * one block per SM with its rows in registers, 3 the three-phase kernel, 0 none
+ * yet.  For tests, which name the form they mean. */
+int GCGE_TestBlockPCGForm(void);
+/* This thread's block CG launches take 1 / workers of the SMs, as a server's
+ * worker's do (0: all of them); returns the setting before.  For tests. */
+int GCGE_TestBlockPCGShare(int workers);
 /* B-orthonormalise columns [start, *end) of x against [0, start) (B NULL =
  * identity), as MultiVecOrth does (src/ops_orth.c:203-394); *end shrinks by
  * the number of dependent columns dropped. */
