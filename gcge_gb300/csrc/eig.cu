@@ -381,18 +381,20 @@ static void launch_jacobi_cta(int s, const double *M, int ldm, float2 *log, int 
 // pair slot k of round r is (P_r[k], P_r[m - 1 - k]); after m - 1 rounds P is
 // the identity again.  CTA c owns the slots [c np / kJC, (c + 1) np / kJC) and
 // holds the two full rows (m floats each) of each of its slots.  A round:
-//   (a) every CTA computes all np rotations from the table of the pairs'
-//       a_pp, a_qq and a_pq that the previous round left in its shared memory;
-//   (b) it updates every 2x2 block (own slot i, any slot j) of its rows,
-//       A <- J^T A J, writes the new rows into the other row buffer at the
-//       slots they hold in the next round, which for at most two rows per CTA
-//       is in the neighbouring CTA's shared memory, and the entries that the
-//       next round's rotations need into every CTA's table;
-//   (c) one cluster barrier makes the next buffers and tables complete.
-// The round is bound by the latency of its serial chain, of which a barrier is
-// the longest link: computing the rotations eight times over costs less than
-// the second barrier that sharing them took (whole eigensolve of s = 180 1.55 ms
-// with two barriers, 1.43 with one).
+//   (a) every CTA computes the rotations of its slots and writes them into the
+//       round table of every CTA of the cluster;
+//   (b) after a cluster barrier, each CTA updates every 2x2 block (own slot i,
+//       any slot j) of its rows, A <- J^T A J, and writes the new rows into
+//       the other row buffer at the slots they hold in the next round, which
+//       for at most two rows per CTA is in the neighbouring CTA's shared
+//       memory;
+//   (c) a second cluster barrier makes the next buffers complete.
+// The round is bound by the latency of its serial chain.  A form with one
+// barrier, in which every CTA computed all rotations from a table of the pairs'
+// entries that the block updates of the previous round kept up to date, paid
+// more in the updates than the barrier costs (kernel, one barrier against two:
+// s = 105 978 and 1043 us, 128 1512 and 1451, 180 2452 and 2404, 260 5857 and
+// 4325, 460 17.3 and 13.8 ms).
 // The stopping test is that of k_jacobi32; every CTA sums the per-CTA
 // off-diagonal masses in the same order, so all take the same decision.
 constexpr int kJC = 8;
@@ -403,7 +405,7 @@ __host__ __device__ inline int jc_slots(int np) { return (np + kJC - 1) / kJC; }
 size_t jacobi_cluster_smem_bytes(int s) {
     const int m = jac_m(s), np = m / 2, ks = jc_slots(np);
     return (size_t)np * sizeof(float4) + (size_t)2 * 2 * ks * m * sizeof(float) +
-           (size_t)2 * kJC * 2 * sizeof(float) + (size_t)2 * 3 * np * sizeof(float) + 64;
+           (size_t)2 * kJC * 2 * sizeof(float) + 64;
 }
 
 // index at position i < m1 + 1 of the circle arrangement after r < m1 rounds
@@ -426,14 +428,9 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
     float4 *tab = reinterpret_cast<float4 *>(jsm);          // [np]: c, s, p, q of the round
     float *rows = reinterpret_cast<float *>(tab + np);      // [2][2 ks][m]
     float *red = rows + (size_t)2 * 2 * ks * m;               // [2][kJC][2]
-    float *piv = red + 2 * kJC * 2;                          // [2][3][np]: a_pp, a_qq, a_pq
     __shared__ float wsum[kJacobiThreads / 32][2];
     __shared__ int stop;
-    // each local row in the next round: where it is stored, its slot (2 k for
-    // the top row of slot k, 2 k + 1 for the bottom one), and for a top row its
-    // partner's index
-    __shared__ float *s_dst[2 * kJacMaxLocal];
-    __shared__ int s_slot[2 * kJacMaxLocal], s_partner[2 * kJacMaxLocal];
+    __shared__ float *s_dst[2 * kJacMaxLocal];  // next-round places of the local rows
     const size_t bufsz = (size_t)2 * ks * m;
     const int k0 = (rank * np) / kJC, k1 = ((rank + 1) * np) / kJC, nloc = k1 - k0;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
@@ -447,20 +444,6 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
         rows[(size_t)lr * m + y] = v;
     }
     cl.sync();  // every CTA of the cluster runs before any remote access
-    // entry `what` (0 a_pp, 1 a_qq, 2 a_pq) of slot k, into every CTA's table
-    auto share = [&](int parity, int what, int k, float v) {
-        float *at = piv + ((size_t)parity * 3 + what) * np + k;
-#pragma unroll
-        for (int c = 0; c < kJC; ++c) *cl.map_shared_rank(at, c) = v;
-    };
-    for (int ls = t; ls < nloc; ls += blockDim.x) {
-        const int k = k0 + ls;
-        const float *top = rows + (size_t)(2 * ls) * m;
-        share(0, 0, k, top[k]);
-        share(0, 1, k, top[m + m - 1 - k]);
-        share(0, 2, k, top[m - 1 - k]);
-    }
-    cl.sync();
     int cur = 0, round = 0, sweep = 0, converged = 0;
     for (sweep = 0; sweep < kMaxSweeps && round + m1 <= max_rounds; ++sweep) {
         // off-diagonal mass at the start of the sweep (P = identity again)
@@ -514,14 +497,13 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
         }
         for (int r = 0; r < m1; ++r) {
             const float *R = rows + cur * bufsz;
-            const int par = round & 1, rn = r + 1 == m1 ? 0 : r + 1;
-            // (a) the round's rotations, from the pairs' entries
-            for (int k = t; k < np; k += blockDim.x) {
+            // (a) the rotations of the local slots, into every CTA's table
+            for (int k = k0 + t; k < k1; k += blockDim.x) {
                 const int p = circle_index(k, r, m1), q = circle_index(m - 1 - k, r, m1);
                 float c = 1.0f, sv = 0.0f;
                 if (p < s && q < s) {
-                    const float *pv = piv + (size_t)par * 3 * np + k;
-                    const float app = pv[0], aqq = pv[np], apq = pv[2 * np];
+                    const float *top = R + (size_t)(2 * (k - k0)) * m;
+                    const float app = top[p], aqq = top[m + q], apq = top[q];
                     const float thr = kRotTol * sqrtf(fabsf(app) * fabsf(aqq));
                     if (fabsf(apq) > thr && fabsf(apq) > 1e-30f) {
                         // (an infinite tau^2 gives the rotation 0, as it should)
@@ -532,8 +514,10 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
                         sv = tt * c;
                     }
                 }
-                tab[k] = make_float4(c, sv, __int_as_float(p), __int_as_float(q));
-                if (k >= k0 && k < k1) log[(size_t)round * np + k] = make_float2(c, sv);
+                const float4 e = make_float4(c, sv, __int_as_float(p), __int_as_float(q));
+#pragma unroll
+                for (int o = 0; o < kJC; ++o) *cl.map_shared_rank(tab + k, o) = e;
+                log[(size_t)round * np + k] = make_float2(c, sv);
             }
             // next-round places of the local rows (circle method)
             for (int lr = (int)blockDim.x - 1 - t; lr < 2 * nloc; lr += blockDim.x) {
@@ -548,10 +532,8 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
                 float *d = rows + (size_t)(cur ^ 1) * bufsz +
                            (size_t)(2 * (kn - (o * np) / kJC) + sn) * m;
                 s_dst[lr] = o == rank ? d : cl.map_shared_rank(d, o);
-                s_slot[lr] = 2 * kn + sn;
-                s_partner[lr] = sn == 0 ? circle_index(m - 1 - kn, rn, m1) : -1;
             }
-            __syncthreads();
+            cl.sync();
             // (b) the 2x2 blocks of the local rows, written to the next buffers
             const float inv_np = 1.0f / (float)np;  // b / np exactly: the quotient's
 #pragma unroll 2
@@ -592,15 +574,6 @@ k_jacobi32_cluster(int s, const double *__restrict__ M, int ldm, float2 *__restr
                 dt[qj] = o12;
                 db[pj] = o21;
                 db[qj] = o22;
-                // what the next round's rotations need of these entries
-                const int nt = s_slot[2 * li], nb = s_slot[2 * li + 1];
-                if (ki == j) {
-                    share(par ^ 1, nt & 1, nt >> 1, o11);
-                    share(par ^ 1, nb & 1, nb >> 1, o22);
-                }
-                const int pt = s_partner[2 * li], pb = s_partner[2 * li + 1];
-                if (pt == pj || pt == qj) share(par ^ 1, 2, nt >> 1, pt == pj ? o11 : o12);
-                if (pb == pj || pb == qj) share(par ^ 1, 2, nb >> 1, pb == pj ? o21 : o22);
             }
             cl.sync();
             cur ^= 1;
