@@ -133,7 +133,7 @@ struct TcArgs {
     int M, N, K;
     const double *A;  // gram: Q (k, r) at A[k + r lda]; lincomb: X (r, k) at A[r + k lda]
     size_t lda;
-    int super_k;      // k per exponent window (gram: a multiple of kTcDrainK)
+    int super_k;      // k per exponent window (gram: a multiple of kTcStageK)
     int kchunk;       // gram: k per work item (multiple of super_k)
     int items;        // work items
     int mtiles, ntiles;
@@ -1295,11 +1295,12 @@ void tc_gram(int n, int m, int w, const double *Q, int ldq, const double *P, int
     a.ntiles = (w + bn - 1) / bn;
     const int mn = a.mtiles * a.ntiles;
     const int sms = device_sms();
-    // one wave of one CTA per SM over all work items (k ranges of a multiple
-    // of the drain chunk), fewer and longer ranges until the partials fit
-    // the scratch
+    // one wave of one CTA per SM over all work items (k ranges of whole stages:
+    // of whole drain chunks, 134 k of a short contraction became 256, and half of
+    // the SMs had no item: 2000 x 200 x 200 44 -> 52 us against 144-k chunks),
+    // fewer and longer ranges until the partials fit the scratch
     int z = std::max(1, sms / mn);
-    long long kc = ((long long)(n + z - 1) / z + kTcDrainK - 1) / kTcDrainK * kTcDrainK;
+    long long kc = ((long long)(n + z - 1) / z + kTcStageK - 1) / kTcStageK * kTcStageK;
     GCGE_REQUIRE((size_t)m * w <= scratch_elems, GCGE_ERR_ARG, "tc_gram: scratch too small");
     while ((size_t)((n + kc - 1) / kc) * m * w > scratch_elems) kc *= 2;
     // the exponent window: the whole k range of a work item, or windows of
