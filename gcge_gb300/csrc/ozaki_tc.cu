@@ -1151,7 +1151,14 @@ __global__ void __launch_bounds__(256) k_tc_reduce(const double *__restrict__ pa
     }
 }
 
-int tc_bn(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : 48); }
+// Column tile of a right operand of n columns: as many tiles as 48-column ones
+// take, of even width (60 columns: two of 32, whose accumulators fit tensor memory
+// twice, instead of 48 + 12 in two of 48; 262144 x 40 -> 60 321 us with 16-k stages,
+// 357 with two of 48, 249).
+int tc_bn(int n) {
+    const int tiles = std::max(1, (n + 47) / 48), w = (n + tiles - 1) / tiles;
+    return w <= 16 ? 16 : (w <= 32 ? 32 : 48);
+}
 
 template <int BN, bool GRAM>
 void launch_tc(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &a, int grid,

@@ -1,6 +1,6 @@
 """The digit products where their work is divided: k ranges of whole 32-k stages (one
 stage, an odd number, a range that ends inside a drain chunk, fewer rows than a
-stage) and several row and column tiles.
+stage), several row and column tiles, and right operands of 49 to 64 columns.
 
 Bound, entry by entry: a product of two truncated operands is off by less than
 2 x 2^-55 x 2 of the largest |x||y| of its row and column (the exponents are
@@ -33,3 +33,15 @@ def test_gram_ranges(gpu_lib, n, m, w):
     got = gpu_lib.dense_gram(Q, R, emulated=True)
     check(got, Q.astype(EXT).T @ R.astype(EXT), n, np.abs(Q).max(0), np.abs(R).max(0),
           np.abs(Q).T @ np.abs(R))
+
+
+@pytest.mark.parametrize("n,k,m", [
+    (130, 8, 49), (1000, 40, 50), (3000, 60, 64), (2050, 144, 60), (5000, 433, 57), (20002, 33, 63)])
+def test_lincomb_of_two_even_column_tiles(gpu_lib, n, k, m):
+    rng = np.random.default_rng(n + k + m)
+    X, C, Y = (rng.standard_normal(s) for s in ((n, k), (k, m), (n, m)))
+    beta = rng.standard_normal(m)
+    got = gpu_lib.dense_lincomb(X, C, Y, beta=beta, alpha=-1.0, emulated=True)
+    exact = Y.astype(EXT) * beta.astype(EXT) - X.astype(EXT) @ C.astype(EXT)
+    check(got, exact, k, np.abs(X).max(1), np.abs(C).max(0),
+          np.abs(X) @ np.abs(C) + np.abs(Y * beta))
