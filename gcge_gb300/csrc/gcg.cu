@@ -557,15 +557,15 @@ int bgs_orth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int star
 // ---------------------------------------------------------------- the solve
 // The FP32 part of a mixed inner solve: CG from 0 on S d = r (r in c.r64, S's FP32
 // values formed), x += d accumulated in FP64, but for the columns of d that left
-// FP32's range (c.pcg.h_out, once the stream has passed).
+// FP32's range (*report, page-locked and zeroed by the caller, gets their bits).
 void mixed_correction(SolverCtx &c, int n, int k, double *x, int ldx, int max_iter, double rate,
-                      double tol, bool rel, cudaStream_t st) {
+                      double tol, bool rel, cudaStream_t st, unsigned long long *report) {
     const int kp = rows_width(k, 4);
     col_to_rows<double, float>(n, k, kp, c.r64.p, c.ld, c.br32.p, st);
     block_pcg_rows<float>(c.pcg, c.upat, c.us32.p, c.br32.p, c.xr32.p, c.rr32.p, c.pr32.p,
                           c.wr32.p, kp, k, max_iter, rate, tol, rel, true, st);
     rows_to_col<float, double>(n, k, kp, c.xr32.p, x, ldx, true, st, &c.pcg.sync.p->out_of_range,
-                               c.pcg.h_out.p);
+                               report);
 }
 
 struct GcgRun {
@@ -951,7 +951,8 @@ struct GcgRun {
     // BlockPCG on S x = b (b in c.bbuf, S = A + sigma B on the union pattern,
     // its values already formed) for bsz columns, starting from and overwriting
     // x (V columns, leading dimension ld).
-    void w_solve(double *x, int bsz, bool mixed, bool have_sx = false) {
+    // `report`: the columns left out of a mixed solve are for check_corrections.
+    void w_solve(double *x, int bsz, bool mixed, bool have_sx = false, bool report = true) {
         if (bsz <= 0) return;
         const bool rel = std::strcmp(g.compW_cg_tol_type, "rel") == 0;
         if (!mixed) {
@@ -972,8 +973,10 @@ struct GcgRun {
                 spmm_calls++;
             }
             axpby(n, bsz, 1.0, c.bbuf.p, ld, -1.0, c.r64.p, ld, st);
+            // (CheckConvergence waited for the stream: no kernel writes the word now)
+            if (report) *c.pcg.h_out.p = 0;
             mixed_correction(c, n, bsz, x, ld, g.compW_cg_max_iter, g.compW_cg_rate,
-                             g.compW_cg_tol, rel, st);
+                             g.compW_cg_tol, rel, st, report ? c.pcg.h_out.p : nullptr);
         }
     }
 
@@ -1050,7 +1053,7 @@ struct GcgRun {
         shift_values(c.upat.padded, c.ua.p, c.ub.p, sigma, c.us64.p, mixed ? c.us32.p : nullptr,
                      st);
         timer.mark(PH_LINSOL);
-        w_solve(colp(V, startW), bsz, mixed);
+        w_solve(colp(V, startW), bsz, mixed, false, false);
         endW = startW + bsz;
         copy_cols(n, bsz, colp(V, startW), ld, colp(V, endW), ld, st);
         w_solve(colp(V, endW), bsz, mixed);

@@ -76,7 +76,7 @@ int bgs_orth(SolverCtx &c, SparseMat *B, double *x, int ldx, int nrows, int star
              bool useB, double zero_tol, int max_reorth, int block_size, int *spmm_calls);
 // The FP32 part of a mixed solve's inner solve (x += d, S d = r64 by block CG).
 void mixed_correction(SolverCtx &c, int n, int k, double *x, int ldx, int max_iter, double rate,
-                      double tol, bool rel, cudaStream_t st);
+                      double tol, bool rel, cudaStream_t st, unsigned long long *report);
 // Union pattern of A, B (B NULL = identity) and the diagonal, with A's and B's
 // values on it; cached on the context by matrix identity.
 void prepare_union(SolverCtx &c, SparseMat *A, SparseMat *B, cudaStream_t st);

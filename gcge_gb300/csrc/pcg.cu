@@ -36,9 +36,9 @@ k_col_to_rows(int n, int k, int kp, const S *__restrict__ X, int ldx, T *__restr
     }
 }
 // *out |= a bit for each column of X (slice-blocked, FP32) with an entry that is
-// not finite.  X once at HBM speed; a kernel of its own, as the solve's kernels
-// have no register left for it (k_block_pcg<float, 20> spilled 36 bytes
-// instead of 20).
+// not finite.  X once at HBM speed (55 us of a 25 ms solve at 128^3 x 40); a
+// kernel of its own, as the three-phase kernel has no register left for it
+// (k_block_pcg<float, 20> spilled 36 bytes instead of 20).
 __global__ void __launch_bounds__(256)
 k_out_of_range(int n, int kp, const float *__restrict__ X, unsigned long long *out) {
     const int G = kp / 4, lane = threadIdx.x & 31;
@@ -64,7 +64,7 @@ k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, 
               const unsigned long long *skip, unsigned long long *report) {
     constexpr int L = 16 / (int)sizeof(T);
     const unsigned long long out = skip ? *skip : 0ull;
-    if (report && blockIdx.x == 0 && threadIdx.x == 0) *report = out;
+    if (report && out && blockIdx.x == 0 && threadIdx.x == 0) *report = out;
     const int G = kp / L, used = (k + L - 1) / L, lane = threadIdx.x & 31;
     const long long units = (long long)((n + 31) / 32) * used;
     for (long long w = blockIdx.x * 8ll + (threadIdx.x >> 5); w < units; w += gridDim.x * 8ll) {
@@ -85,6 +85,13 @@ k_rows_to_col(int n, int k, int kp, const T *__restrict__ X, D *__restrict__ Y, 
     }
 }
 
+void mark_out_of_range(int n, int kp, const float *X, unsigned long long *out, cudaStream_t st) {
+    const long long units = (long long)((n + 31) / 32) * (kp / 4);
+    const int g = (int)std::max(1ll, std::min((units + 7) / 8, 16ll * device_sms()));
+    k_out_of_range<<<g, 256, 0, st>>>(n, kp, X, out);
+    GCGE_CHECK_LAUNCH();
+    count_launch();
+}
 template <typename S, typename T>
 void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t st) {
     const long long units = (long long)((n + 31) / 32) * (kp / (16 / (int)sizeof(T)));
@@ -95,17 +102,10 @@ void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t s
 }
 template <typename T, typename D>
 void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st,
-                 unsigned long long *out, unsigned long long *report) {
+                 const unsigned long long *out, unsigned long long *report) {
     constexpr int L = 16 / (int)sizeof(T);
     const long long units = (long long)((n + 31) / 32) * ((k + L - 1) / L);
     const int g = (int)std::max(1ll, std::min((units + 7) / 8, 16ll * device_sms()));
-    if constexpr (sizeof(T) == 4) {
-        if (out) {
-            k_out_of_range<<<g, 256, 0, st>>>(n, kp, X, out);
-            GCGE_CHECK_LAUNCH();
-            count_launch();
-        }
-    }
     k_rows_to_col<T, D><<<g, 256, 0, st>>>(n, k, kp, X, Y, ldy, add ? 1 : 0, out, report);
     GCGE_CHECK_LAUNCH();
     count_launch();
@@ -113,9 +113,9 @@ void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cuda
 template void col_to_rows<double, double>(int, int, int, const double *, int, double *, cudaStream_t);
 template void col_to_rows<double, float>(int, int, int, const double *, int, float *, cudaStream_t);
 template void rows_to_col<double, double>(int, int, int, const double *, double *, int, bool,
-                                          cudaStream_t, unsigned long long *, unsigned long long *);
+                                          cudaStream_t, const unsigned long long *, unsigned long long *);
 template void rows_to_col<float, double>(int, int, int, const float *, double *, int, bool,
-                                         cudaStream_t, unsigned long long *, unsigned long long *);
+                                         cudaStream_t, const unsigned long long *, unsigned long long *);
 
 void PcgWork::timing_reset(cudaStream_t st) {
     ev_used = 0;

@@ -26,7 +26,7 @@ struct PcgSync {
     unsigned long long arrive;  // block arrivals at barriers, over the launch
     int error;                  // a barrier wait ran out of time
     int pad;
-    unsigned long long out_of_range;  // columns rows_to_col found not finite, a bit each
+    unsigned long long out_of_range;  // FP32: columns of x that are not finite, a bit each
 };
 struct PcgStats {
     double kernel_bytes;         // algorithmic bytes of the whole solves
@@ -46,7 +46,8 @@ struct PcgWork {
     DevBuf<PcgStats> stats;
     PinnedBuf<PcgScalars> h_sc;
     PinnedBuf<PcgStats> h_stats;
-    PinnedBuf<unsigned long long> h_out;  // columns rows_to_col left out, a bit each
+    // columns rows_to_col left out, a bit each; cleared before the launch
+    PinnedBuf<unsigned long long> h_out;
     // whole-kernel timing (event pairs) and algorithmic bytes of the solves
     std::vector<cudaEvent_t> ev;
     size_t ev_used = 0;
@@ -62,7 +63,8 @@ struct PcgWork {
 
 // Solve S x = b column-wise (S on the SELL pattern `pat` with values sval)
 // starting from x (or from 0 when x_zero, in which case x need not be
-// initialised).  B, X, R, P, W are slice-blocked n x kp blocks
+// initialised).  In FP32 and from 0, wk.sync->out_of_range gets a bit for each
+// column of x that is not finite.  B, X, R, P, W are slice-blocked n x kp blocks
 // (pcg_block_elems; padding rows and columns of B and X zero).  One persistent launch runs the
 // whole iteration; the iteration count and any error stay on the device
 // (PcgWork::collect, or pcg_last_iters after a synchronisation).
@@ -94,11 +96,12 @@ inline size_t pcg_block_elems(int n, int kp) { return (size_t)((n + 31) / 32) * 
 // Column-major (ld) <-> slice-blocked (kp) block conversions (pcg.cu).
 template <typename S, typename T>
 void col_to_rows(int n, int k, int kp, const S *X, int ldx, T *Y, cudaStream_t st);
-// add: Y += X.  With `out` (FP32; a zeroed word in device memory) the columns of X
-// that are not finite are left out, whole, and have a bit each in *out and in
-// *report (page-locked memory).
+// add: Y += X.  The columns whose bit in *out (device memory) is set are left out,
+// whole; *report (page-locked memory) gets the bits when there are any.
 template <typename T, typename D>
 void rows_to_col(int n, int k, int kp, const T *X, D *Y, int ldy, bool add, cudaStream_t st,
-                 unsigned long long *out = nullptr, unsigned long long *report = nullptr);
+                 const unsigned long long *out = nullptr, unsigned long long *report = nullptr);
+// *out |= a bit for each column of the FP32 block X that is not finite.
+void mark_out_of_range(int n, int kp, const float *X, unsigned long long *out, cudaStream_t st);
 
 }  // namespace gcge

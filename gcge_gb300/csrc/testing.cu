@@ -100,7 +100,8 @@ int GCGE_MixedInnerSolve(void *A, void *B, double sigma, void **b, void **x, int
         shift_values(c.upat.padded, c.ua.p, c.ub.p, sigma, c.us64.p, c.us32.p, st);
         spmm<double>(c.upat, c.us64.p, xv->data, xv->ld, c.r64.p, c.ld, k, st);
         axpby(n, k, 1.0, bv->data, bv->ld, -1.0, c.r64.p, c.ld, st);
-        mixed_correction(c, n, k, xv->data, xv->ld, max_iter, rate, tol, false, st);
+        mixed_correction(c, n, k, xv->data, xv->ld, max_iter, rate, tol, false, st,
+                         c.pcg.h_out.p);
         const int it = pcg_last_iters(c.pcg, st);
         if (iters) *iters = it;
         if (out_of_range) *out_of_range = *c.pcg.h_out.p;
