@@ -522,8 +522,8 @@ __device__ __forceinline__ void cur_next(const TcArgs &a, TcCursor &c) {
 // held: they reach only output rows (or columns) that are not read.
 //
 // The workers bound it, by their instructions (half of the issue slots, the ALU
-// at 52%) and their latency at four warps per scheduler; the tensor cores are
-// busy a quarter of the time, HBM a third.  So a stage is as long as shared
+// at 51%) and their latency at four warps per scheduler; the tensor cores are
+// busy a quarter of the time, HBM 23% (524288 x 360 x 40, 0.92 ms).  So a stage is as long as shared
 // memory allows (a third of the instructions of 16-k stages were waits, cursors
 // and addresses), the code is short (a second copy of the conversion cost 5% in
 // instruction fetches) and no register is spilled in the loop (the shared memory
@@ -1081,7 +1081,7 @@ __global__ void __launch_bounds__(256) k_tc_exprows(const double *__restrict__ X
 
 // Right operand of a linear combination (C, K x N, element (k, c) at
 // C[k + c ldc]) prepared once per call: block (window, n tile) writes the
-// exponent fields of its BN columns and the digit planes of each 16-k digit
+// exponent fields of its BN columns and the digit planes of each 32-k digit
 // stage of the window in the stage layout of the product kernel.
 template <int BN>
 __global__ void __launch_bounds__(256) k_tc_bprep(const double *__restrict__ C, size_t ldc, int N,
@@ -1302,12 +1302,17 @@ void tc_gram(int n, int m, int w, const double *Q, int ldq, const double *P, int
     a.ntiles = (w + bn - 1) / bn;
     const int mn = a.mtiles * a.ntiles;
     const int sms = device_sms();
-    // one wave of one CTA per SM over all work items (k ranges of whole stages:
-    // of whole drain chunks, 134 k of a short contraction became 256, and half of
-    // the SMs had no item: 2000 x 200 x 200 44 -> 52 us against 144-k chunks),
-    // fewer and longer ranges until the partials fit the scratch
+    // one wave of one CTA per SM over all work items, fewer and longer k ranges
+    // until the partials fit the scratch.  Ranges are whole drain chunks, and
+    // whole stages where several tiles share the SMs, whose short ranges a rounding
+    // to chunks may double (2000 x 200 x 200: 134 k became 256 and half of the SMs had
+    // no item, 52 us, with stages 42; 144-k chunks 44).  With one tile, shorter
+    // ranges make a lone short product faster (4160 x 4 x 4 13.1 -> 8.4 us) but
+    // take more of the part from other streams: a batch of 256 mixed solves by 8
+    // workers 7.46 -> 7.51 s.
     int z = std::max(1, sms / mn);
-    long long kc = ((long long)(n + z - 1) / z + kTcStageK - 1) / kTcStageK * kTcStageK;
+    const int unit = mn > 1 ? kTcStageK : kTcDrainK;
+    long long kc = ((long long)(n + z - 1) / z + unit - 1) / unit * unit;
     GCGE_REQUIRE((size_t)m * w <= scratch_elems, GCGE_ERR_ARG, "tc_gram: scratch too small");
     while ((size_t)((n + kc - 1) / kc) * m * w > scratch_elems) kc *= 2;
     // the exponent window: the whole k range of a work item, or windows of
