@@ -31,8 +31,10 @@
 // scattered rows.  T = double (FP64 GCG) or float (mixed precision: FP32
 // values and FP32 accumulation within a block; cross-block sums in double).
 //
-// Every barrier wait is bounded (time and poll count); a wait that runs out
-// sets an error flag that makes all blocks return, and the host reports it.
+// Every grid-barrier wait is bounded (time and poll count); a wait that runs out
+// sets an error flag that makes all blocks return, and the host reports it.  The
+// cluster form below waits at the hardware's cluster barrier, which has no bound:
+// the cluster's blocks are scheduled together and wait for nobody else.
 //
 // Small operators, whose steps are bound by the barriers and by the latency of
 // each phase instead, run k_pcg_small (below).
@@ -675,11 +677,14 @@ k_block_pcg(PcgArgs<T> a) {
 #pragma unroll
             for (int u = 0; u < G; ++u) ga[u] = s_gact[u] != 0;
             // FP32, while every group is active: two entries' loads in flight per
-            // lane instead of one's (30 steps, 64^3 27-point: k = 8 1498 -> 1178 us,
-            // k = 28 4070 -> 3444; 72^3 7-point: 825 -> 789, 3629 -> 3415).  Not at 16
-            // and 20 columns, whose 64 registers are few for the loads (72^3, k = 20
-            // 2116 -> 2135; 64^3 27-point 2568 -> 2401), nor in FP64, which its FMAs
-            // bound.
+            // lane instead of one's (30 steps, one entry against two: 64^3 27-point
+            // k = 8 1335 and 1066 us, k = 28 4071 and 3452; 72^3 7-point 774 and 768,
+            // 3596 and 3398).  At 16 and 20 columns the 64 registers are few for the
+            // loads, and the operator decides: 700^2 5-point k = 16 1954 and 2014 us,
+            // k = 20 2633 and 2721; 72^3 7-point 1551 and 1581, 2100 and 2116; 64^3
+            // 27-point 2068 and 2020, 2467 and 2354; 128^3 7-point k = 20 12.5 and 11.7
+            // ms.  Operators of few entries per row are the common ones: one entry.
+            // Not in FP64, which its FMAs bound.
             constexpr bool two_entries = sizeof(T) == 4 && (KP < 16 || KP > 20);
             bool all_active = true;
 #pragma unroll

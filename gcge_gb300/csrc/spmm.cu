@@ -161,8 +161,10 @@ k_residual(const long long *__restrict__ sa, const int *__restrict__ ca,
 
 constexpr int kMaxChunk = 40;
 
-// Width class of a launch of kc columns for the tuner: candidates within one
-// class differ too little in registers to be worth timing.
+// Width class of a launch of kc columns for the tuner, which tries one split per
+// class (the one of fewest launches): every trial costs four SpMMs.  The classes
+// are wider than the kernel's register widths; whether a trial per width would
+// find better splits has not been measured.
 static int spmm_dispatch_width(int kc) {
     return kc <= 4 ? 4 : kc <= 8 ? 8 : kc <= 16 ? 16 : kc <= 24 ? 24 : kc <= 32 ? 32 : 40;
 }

@@ -7,13 +7,14 @@ columns, blocks of bs = 20).
     python tests/profile_cases.py both
     python tests/profile_cases.py pcg       # FP32 block PCG, 20 columns, 30 steps
     python tests/profile_cases.py eig       # dense eigensolver, s = 200
-    python tests/profile_cases.py pcgsmall  # FP32 block PCG, 2D n = 4160 (cluster form)
+    python tests/profile_cases.py pcgsmall  # FP32 block PCG, 2D n = 4160 (k_pcg_small)
     python tests/profile_cases.py pcg128    # FP32 block PCG, 128^3 variable coefficient, 40 columns
 
 Each case runs the FP64-accurate digit-plane product once after one warm-up
 call, through the same C-ABI entry points the parity tests use
 (GCGE_DenseGram / GCGE_DenseLinComb), and checks the result against the FP64
-kernel's.  Under ncu, select the product kernel with -k regex:k_oz_gemm.
+kernel's.  Under ncu, select the product kernel with -k regex:k_tc_digits, the
+FP64 ones with -k regex:k_gram_chunk or k_lincomb.
 
 The pcg case runs the persistent FP32 block PCG of the W step (30 CG steps,
 no early stop) on the shifted generalized 64^3 operator A + sigma B through
@@ -22,7 +23,8 @@ dropped; select it with -k regex:k_block_pcg.
 
 The pcgsmall case runs the same solve on a batch-sized operator (anisotropic
 2D 64 x 65, diagonal B, n = 4160, 130 slices), which the library runs in the
-kernel's cluster form (one thread-block cluster, hardware barrier).
+small operators' kernel (one block per SM at 20 columns); select it with -k
+regex:k_pcg_small.
 
 The eig case runs the dense eigensolver of the Rayleigh-Ritz step
 (GCGE_DenseEig) on a 200 x 200 matrix shaped like a late GCG projection (a
